@@ -157,18 +157,19 @@ __device__ __forceinline__ uint32_t e2m1_code_sr(float v, float u) {
 }
 
 // ---------------------------------------------------------------------------------------------- device: division
-// x / y rounded to nearest, from a correctly rounded reciprocal ry = __frcp_rn(y) that the caller shares between many
-// quotients: one product and two residual corrections with fused multiply-adds (the sequence compilers emit for an
-// fp32 division, minus the reciprocal and the range checks). The residuals are exact, so the result is the correctly
-// rounded quotient whenever no intermediate leaves the normal range; outside it the plain division is used.
+// x / y rounded to nearest from ry = RN(1 / y), which the caller shares between the many quotients by one divisor:
+// Markstein's correction ("Computation of elementary functions on the IBM RISC System/6000 processor", IBM Journal of
+// Research and Development 34, 1990; the case of a divisor known in advance: Brisebarre, Muller and Raina, "Accelerating
+// correctly rounded floating-point division when the divisor is known in advance", IEEE Transactions on Computers 53,
+// 2004): the product q = RN(x ry) is off by less than two units in the last place, its residual r = x - y q is formed by
+// one fused multiply-add, and RN(q + r ry) is the correctly rounded quotient. Run over all 2^46 pairs of fp32
+// significands on a B200 it agreed with the plain division on every one; exponents only scale the three operations while
+// nothing leaves the normal range, which the callers (or the check below) establish.
 static __device__ __noinline__ float div_general(float x, float y) { return x / y; }
 
 __device__ __forceinline__ float div_rn(float x, float y, float ry) {
   const float q0 = x * ry;
-  float e = fmaf(-y, q0, x);
-  float q = fmaf(e, ry, q0);
-  e = fmaf(-y, q, x);
-  q = fmaf(e, ry, q);
+  const float q = fmaf(fmaf(-y, q0, x), ry, q0);
   const float aq = fabsf(q0);
   // zero, tiny, huge or non-finite: the general path, kept out of line so that it costs nothing when not taken
   if (__builtin_expect(!(aq > 1e-30f && aq < 1e30f), 0)) return div_general(x, y);
@@ -217,11 +218,8 @@ __device__ __forceinline__ f32x2 prod2p(f32x2 a, f32x2 b) {
 }
 // x / y per lane from ny = -y and ry = rcp_rn(y): div_rn without its range check (the caller establishes the range)
 __device__ __forceinline__ f32x2 div2p(f32x2 x, f32x2 ny, f32x2 ry) {
-  const f32x2 q0 = mul2p(x, ry);
-  f32x2 e = fma2p(ny, q0, x);
-  f32x2 q = fma2p(e, ry, q0);
-  e = fma2p(ny, q, x);
-  return fma2p(e, ry, q);
+  const f32x2 q = mul2p(x, ry);
+  return fma2p(fma2p(ny, q, x), ry, q);
 }
 
 // ---------------------------------------------------------------------------------------------- device: fast E2M1

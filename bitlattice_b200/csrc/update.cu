@@ -260,7 +260,7 @@ struct StepParams {
 //  * (a, latent) of an element depend only on its code nibble and phase bits: shared-memory tables built with the
 //    reference's formula at kernel start replace the per-element level / neighbour / latent arithmetic;
 //  * divisions sharing a divisor (the old and new group scale, a column's denominator, the RMS divisor) go through
-//    one correctly rounded reciprocal per divisor and two fused residual corrections (div_rn);
+//    one correctly rounded reciprocal per divisor and one fused residual correction (div_rn);
 //  * the nearest level comes from the hardware E2M1 conversion (ties to even). The reference breaks ties to the lower
 //    level, but the projection is invariant to that choice: a target exactly half-way between levels L < U gives
 //    (U, phase -half) from either side (from L the phase code reaches +half and carries over), and with 0 phase bits

@@ -342,7 +342,7 @@ enum { BL_GEMM_AUTO = 0, BL_GEMM_TILE = 1, BL_GEMM_PERSISTENT = 2, BL_GEMM_PAIR 
 BL_API int bl_nvfp4_gemm_select(int kernel);
 
 /* Diagnostic, no counterpart in the reference: the kernels replace fp32 divisions that share a divisor by a product
- * with its correctly rounded reciprocal plus two fused residual corrections. This runs that routine against the
+ * with its correctly rounded reciprocal plus one fused residual correction. This runs that routine against the
  * plain division on n pseudo-random operand pairs (synchronously, with a temporary 8-byte device allocation) and
  * stores the number of results that differ in any bit; the test-suite requires 0. */
 BL_API int bl_selftest_division(uint64_t n, uint32_t seed, uint64_t* mismatches, int device);
