@@ -198,6 +198,11 @@ __device__ __forceinline__ f32x2 add2p(f32x2 a, f32x2 b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+__device__ __forceinline__ f32x2 add2p_up(f32x2 a, f32x2 b) {       // rounded toward +infinity
+  f32x2 r;
+  asm("add.rp.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __device__ __forceinline__ f32x2 sub2p(f32x2 a, f32x2 b) {
   f32x2 r;
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));

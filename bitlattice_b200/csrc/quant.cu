@@ -537,54 +537,142 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
   }
 }
 
-// NVFP4 W [N, K] -> NVFP4 of W^T [K, N]; same tiling, the tile holds (level*scale)*global
+// ---- W^T ---------------------------------------------------------------------------------------------------------------
+
+// two E2M1 codes (a byte) -> their levels as a pair of halves (exact)
+__device__ __forceinline__ __half2 e2m1_levels2(uint32_t byte) {
+  uint32_t h2;
+  asm("{\n\t.reg .b8 b;\n\tcvt.u8.u32 b, %1;\n\tcvt.rn.f16x2.e2m1x2 %0, b;\n\t}" : "=r"(h2) : "r"(byte));
+  return *reinterpret_cast<const __half2*>(&h2);
+}
+
+// codes of v[i] / se for the 16 values of a block by plain divisions: scales outside the range of the packed route
+static __device__ __noinline__ uint2 e2m1_nearest_x16_exact(const float* v, float se) {
+  uint32_t w[2] = {0u, 0u};
+  for (int i = 0; i < 16; ++i) w[i >> 3] |= e2m1_code_nearest(v[i] / se) << (4 * (i & 7));
+  return make_uint2(w[0], w[1]);
+}
+
+constexpr int kRqN = 128, kRqK = 128;       // rows and columns of W per CTA
+
+// NVFP4 W [N, K] -> NVFP4 of W^T [K, N], values (level * scale) * global. A thread owns 4 columns of W by one block of 16
+// rows: a row costs it one 16-bit load, two conversions and two packed products, since level * scale is exact in fp16 (7
+// significant bits between 2^-10 and 2688); the block's amax is the fp16 maximum times the global scale, rounding being
+// monotone. Codes and scale bytes leave through shared memory as 32-byte pieces of rows of W^T and 4-byte pieces of the
+// tiled scales.
+//
+// Both factors have few bits, so a quotient v / se sits at a midpoint between two levels for a few percent of the
+// elements: bracketing it and repairing the ties, as the activation quantizers do, had most warps run the repair (12288 x
+// 4096: 122 us, now 38; 25600 x 5120: 302, now 89). Here the quotient is formed exactly and the tie goes to the lower level by arithmetic: with d = 1/8 the
+// midpoints are multiples of d, and ceil(x / d) d - d / 2 lies on the same side of every midpoint as x does, an x at a
+// midpoint counting as below it.
+template <int LAYOUT>
 __global__ void __launch_bounds__(kQThreads) requantize_t_kernel(const uint8_t* __restrict__ wcodes,
                                                                  const uint8_t* __restrict__ wscales,
                                                                  const float* __restrict__ global, int64_t N, int64_t K,
                                                                  uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
-                                                                 float* __restrict__ global_out, int layout) {
-  __shared__ float tile[kTM][kTK + 1];
+                                                                 float* __restrict__ global_out) {
+  __shared__ __half2 s_in[kRqN][kRqK / 16];                 // the rows' block scales, each as a pair
+  __shared__ __align__(16) uint2 s_codes[kRqN / 16][kRqK];
+  __shared__ __align__(16) uint8_t s_scales[kRqK][kRqN / 16];
   const float g = global[0];
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) global_out[0] = g;
-  const int64_t n0 = static_cast<int64_t>(blockIdx.y) * kTM, k0 = static_cast<int64_t>(blockIdx.x) * kTK;
-  // 128 rows x 8 chunks of 8 columns
-  for (int i = threadIdx.x; i < kTM * (kTK / 8); i += kQThreads) {
-    const int rr = i / (kTK / 8), c8 = i % (kTK / 8);
-    const int64_t n = n0 + rr, k = k0 + c8 * 8;
-    if (n < N && k < K) {
-      const uint32_t word = *reinterpret_cast<const uint32_t*>(wcodes + n * (K / 2) + k / 2);
-      const float s = e4m3_decode(wscales[n * (K / 16) + k / 16]);
+  const int64_t n0 = static_cast<int64_t>(blockIdx.y) * kRqN, k0 = static_cast<int64_t>(blockIdx.x) * kRqK;
+  const int lane = threadIdx.x & 31, nb = threadIdx.x >> 5;
+  const int64_t k = k0 + 4 * lane, n = n0 + 16 * nb;        // N and K are multiples of 16: a thread is in or out as a whole
+  const bool active = k < K && n < N;
+  uint32_t raw[16];
+  if (active) {
+    const uint8_t* p = wcodes + n * (K / 2) + k / 2;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) tile[rr][c8 * 8 + j] = level_of_rank(rank_of_code((word >> (4 * j)) & 0xFu)) * s * g;
-    } else {
+    for (int i = 0; i < 16; ++i) raw[i] = *reinterpret_cast<const uint16_t*>(p + i * (K / 2));
+  }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) tile[rr][c8 * 8 + j] = 0.0f;
-    }
+  for (int e = 0; e < kRqN * (kRqK / 16) / kQThreads; ++e) {
+    const int j = e * kQThreads + threadIdx.x, row = j / (kRqK / 16), grp = j % (kRqK / 16);
+    const bool in = n0 + row < N && k0 + 16 * grp < K;
+    s_in[row][grp] = __float2half2_rn(in ? e4m3_decode(wscales[(n0 + row) * (K / 16) + k0 / 16 + grp]) : 0.0f);
   }
   __syncthreads();
-  // one thread per (column k of W, block of 16 rows): lanes walk k, so tile reads are conflict-free
-  const float rg = __frcp_rn(g);
-  for (int it = 0; it < 2; ++it) {
-    const int w = it * kQThreads + threadIdx.x;
-    const int kk = w & (kTK - 1), nb = w >> 6;
-    const int64_t k = k0 + kk, n = n0 + nb * 16;
-    if (!(k < K && n < N)) continue;
-    float v[16];
-    float amax = 0.0f;
+  if (active) {
+    __half2 pr[2][16];                                      // level * scale of columns (k, k + 1) and (k + 2, k + 3)
+    __half2 am[2] = {__float2half2_rn(0.0f), __float2half2_rn(0.0f)};
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      v[i] = tile[nb * 16 + i][kk];
-      amax = fmaxf(amax, fabsf(v[i]));
+      const __half2 s = s_in[16 * nb + i][lane >> 2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        pr[c][i] = __hmul2(e2m1_levels2((raw[i] >> (8 * c)) & 0xFFu), s);
+        am[c] = __hmax2(am[c], __habs2(pr[c][i]));
+      }
     }
-    // the reference kernel's own block rule for W^T (csrc/act_quant.cu:66-86): scale amax/6/g, s > 0 ? v/s : 0
-    const uint32_t sb = e4m3_encode(div_rn(div_rn(amax, 6.0f, kInv6), g, rg));
-    const float se = e4m3_decode(sb) * g;
-    const uint2 out = se > 0.0f ? e2m1_rtn16(v, 1.0f, se, rcp_approx(se)) : make_uint2(0u, 0u);
-    *reinterpret_cast<uint2*>(codes + k * (N / 2) + n / 2) = out;
-    scales[scale_index(layout, k, n / 16, N / 16)] = static_cast<uint8_t>(sb);
+    const float rg = __frcp_rn(g);
+    uint2 out[4];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      // the reference kernel's own block rule for W^T (csrc/act_quant.cu:66-86): scale amax/6/g, s > 0 ? v/s : 0
+      float amax[2], se[2];
+      const float2 amf = __half22float2(am[c]);
+      amax[0] = amf.x * fabsf(g);
+      amax[1] = amf.y * fabsf(g);
+      bool ok = true;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t sb = e4m3_encode(div_rn(div_rn(amax[e], 6.0f, kInv6), g, rg));
+        se[e] = e4m3_decode(sb) * g;
+        s_scales[4 * lane + 2 * c + e][nb] = static_cast<uint8_t>(sb);
+        ok = ok && se[e] > 1e-28f && se[e] < 1e28f && amax[e] < 1e28f;     // quotients of normal numbers (div2p)
+      }
+      float y[2][16];
+      if (__builtin_expect(ok, 1)) {
+        const f32x2 g2 = pk(g, g), nse2 = pk(-se[0], -se[1]), rse2 = pk(__frcp_rn(se[0]), __frcp_rn(se[1]));
+        constexpr float kM = 1572864.0f;                    // 1.5 * 2^20: a sum with it has ulp 1/8
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float2 p = __half22float2(pr[c][i]);
+          const f32x2 x = div2p(mul2p(pk(p.x, p.y), g2), nse2, rse2);
+          const f32x2 up = add2p_up(x, pk(kM, kM));
+          upk(add2p(add2p(up, pk(-kM, -kM)), pk(-0.0625f, -0.0625f)), y[0][i], y[1][i]);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          out[2 * c + e] = make_uint2(e2m1_drop_negative_zero(cvt_e2m1x8_merged(y[e])),
+                                      e2m1_drop_negative_zero(cvt_e2m1x8_merged(y[e] + 8)));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float2 p = __half22float2(pr[c][i]);
+          y[0][i] = p.x * g;
+          y[1][i] = p.y * g;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          out[2 * c + e] = se[e] > 0.0f ? e2m1_nearest_x16_exact(y[e], se[e]) : make_uint2(0u, 0u);
+      }
+    }
+    uint4* dst = reinterpret_cast<uint4*>(&s_codes[nb][4 * lane]);
+    dst[0] = make_uint4(out[0].x, out[0].y, out[1].x, out[1].y);
+    dst[1] = make_uint4(out[2].x, out[2].y, out[3].x, out[3].y);
+  }
+  __syncthreads();
+  // write-out: thread -> (row of W^T, four of its eight blocks)
+  const int row = threadIdx.x >> 1, b0 = (threadIdx.x & 1) * 4;
+  const int64_t kr = k0 + row, nn = n0 + 16 * b0, cols16 = N / 16;
+  if (kr >= K || nn >= N) return;
+  uint2* dst = reinterpret_cast<uint2*>(codes + kr * (N / 2) + nn / 2);
+  if (nn + 64 <= N && (cols16 & 3) == 0) {                   // rows of whole 32-byte pieces: the usual case
+    const uint2 c0 = s_codes[b0][row], c1 = s_codes[b0 + 1][row], c2 = s_codes[b0 + 2][row], c3 = s_codes[b0 + 3][row];
+    reinterpret_cast<uint4*>(dst)[0] = make_uint4(c0.x, c0.y, c1.x, c1.y);
+    reinterpret_cast<uint4*>(dst)[1] = make_uint4(c2.x, c2.y, c3.x, c3.y);
+    *reinterpret_cast<uint32_t*>(scales + scale_index(LAYOUT, kr, nn / 16, cols16)) =
+        *reinterpret_cast<const uint32_t*>(&s_scales[row][b0]);
+  } else {
+    for (int e = 0; e < 4 && nn + 16 * e < N; ++e) {
+      dst[e] = s_codes[b0 + e][row];
+      scales[scale_index(LAYOUT, kr, nn / 16 + e, cols16)] = s_scales[row][b0 + e];
+    }
   }
 }
-
 
 // ------------------------------------------------------------------------------------------------ dequantize, layout
 
@@ -610,13 +698,36 @@ __global__ void __launch_bounds__(kQThreads) dequantize_kernel(const uint8_t* __
   }
 }
 
+// Row-major scales -> 128x4 tiles. WORD: rows of whole 32-bit words (cols16 % 4 == 0, 4-byte aligned source): a word is
+// four neighbouring scales of a row and one contiguous piece of a tile. The CTA's threads walk the output, 512-byte tiles
+// whole, so stores are full lines; a thread's four loads go to rows 32 apart. (Byte by byte with a 64-bit division each, 25600 x 320
+// scales took 23 us, now 9.)
+template <bool WORD>
 __global__ void to_blocked_kernel(const uint8_t* __restrict__ scales, int64_t rows, int64_t cols16,
                                   uint8_t* __restrict__ out) {
-  const int64_t n = rows * cols16;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / cols16, c = i - r * cols16;
-    out[scale_index(BL_SF_BLOCKED, r, c, cols16)] = scales[i];
+  if constexpr (WORD) {
+    const int64_t nc = cols16 >> 2;
+    const int64_t tiles = ((rows + 127) >> 7) * nc;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(scales);
+    const int r32 = threadIdx.x & 31, warps = blockDim.x >> 5;
+    for (int64_t t = static_cast<int64_t>(blockIdx.x) * warps + (threadIdx.x >> 5); t < tiles;
+         t += static_cast<int64_t>(gridDim.x) * warps) {
+      const int64_t rb = t / nc, c = t - rb * nc;
+      uint32_t w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int64_t r = rb * 128 + 32 * q + r32;
+        w[q] = r < rows ? src[r * nc + c] : 0u;
+      }
+      reinterpret_cast<uint4*>(out + t * 512)[r32] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  } else {
+    const int64_t n = rows * cols16;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+      const int64_t r = i / cols16, c = i - r * cols16;
+      out[scale_index(BL_SF_BLOCKED, r, c, cols16)] = scales[i];
+    }
   }
 }
 
@@ -841,9 +952,11 @@ extern "C" int bl_nvfp4_requantize_t(const uint8_t* codes, const uint8_t* scales
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (sf_layout == BL_SF_BLOCKED && blocked_needs_padding(K, N / 16))
     BL_CUDA(cudaMemsetAsync(out_scales, 0, bl_blocked_scale_bytes(K, N / 16), st));
-  const dim3 grid(static_cast<unsigned>((K + kTK - 1) / kTK), static_cast<unsigned>((N + kTM - 1) / kTM));
-  requantize_t_kernel<<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, N, K, out_codes, out_scales, global_out,
-                                                  sf_layout);
+  const dim3 grid(static_cast<unsigned>((K + kRqK - 1) / kRqK), static_cast<unsigned>((N + kRqN - 1) / kRqN));
+  if (sf_layout == BL_SF_BLOCKED)
+    requantize_t_kernel<BL_SF_BLOCKED><<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, N, K, out_codes, out_scales, global_out);
+  else
+    requantize_t_kernel<BL_SF_ROWMAJOR><<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, N, K, out_codes, out_scales, global_out);
   BL_CUDA(cudaGetLastError());
   return 0;
 }
@@ -874,8 +987,13 @@ extern "C" int bl_nvfp4_scales_to_blocked(const uint8_t* scales, int64_t rows, i
   BL_REQUIRE(scales && out && rows > 0 && cols16 > 0, "scales_to_blocked: null or empty input");
   BL_DEVICE(device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (blocked_needs_padding(rows, cols16)) BL_CUDA(cudaMemsetAsync(out, 0, bl_blocked_scale_bytes(rows, cols16), st));
-  to_blocked_kernel<<<grid_for(rows * cols16, kQThreads, device), kQThreads, 0, st>>>(scales, rows, cols16, out);
+  if (cols16 % 4 == 0 && (reinterpret_cast<uintptr_t>(scales) & 3u) == 0 && aligned16(out)) {
+    const int64_t tiles = ((rows + 127) / 128) * (cols16 / 4);
+    to_blocked_kernel<true><<<grid_for(tiles * 32, kQThreads, device), kQThreads, 0, st>>>(scales, rows, cols16, out);
+  } else {
+    if (blocked_needs_padding(rows, cols16)) BL_CUDA(cudaMemsetAsync(out, 0, bl_blocked_scale_bytes(rows, cols16), st));
+    to_blocked_kernel<false><<<grid_for(rows * cols16, kQThreads, device), kQThreads, 0, st>>>(scales, rows, cols16, out);
+  }
   BL_CUDA(cudaGetLastError());
   return 0;
 }
