@@ -147,11 +147,8 @@ __device__ __forceinline__ float fos_candidate(const float v[16], float se, uint
 // kModeRtn: reference.quantize 'rtn'. kModeSr: fp4ref.quantize 'sr' (idx0 = flat index of v[0]). kModeFosMse /
 // kModeFosMae: fp4ref.quantize 'rtn' with four_over_six (pre must be 1).
 template <int MODE>
-__device__ __forceinline__ uint2 quantize_block(const float v[16], float pre, float g, float rg, uint32_t key,
+__device__ __forceinline__ uint2 quantize_block(const float v[16], float amax, float pre, float g, float rg, uint32_t key,
                                                 uint32_t idx0, uint32_t* scale) {
-  float amax = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
   amax *= pre;
   if constexpr (MODE == kModeRtn) {
     const uint32_t sb = e4m3_encode(div_rn(fmaxf(div_rn(amax, 6.0f, kInv6), 1e-12f), g, rg));
@@ -186,6 +183,20 @@ template <typename T>
 __device__ __forceinline__ void load_raw16(const T* p, Raw16<T>& r) {
 #pragma unroll
   for (int i = 0; i < static_cast<int>(sizeof(T)); ++i) r.q[i] = __ldcs(reinterpret_cast<const uint4*>(p) + i);
+}
+
+// max |element|: the 16-bit types two at a time, without unpacking
+template <typename T>
+__device__ __forceinline__ float max_abs_raw16(const Raw16<T>& r, const float v[16]) {
+  if constexpr (sizeof(T) == 4) return max_abs16(v);
+  else {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(r.q);
+    using T2 = typename std::conditional<std::is_same<T, __nv_bfloat16>::value, __nv_bfloat162, __half2>::type;
+    T2 m = __habs2(*reinterpret_cast<const T2*>(&w[0]));
+#pragma unroll
+    for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const T2*>(&w[i])));
+    return fmaxf(to_f<T>(m.x), to_f<T>(m.y));
+  }
 }
 
 template <typename T>
@@ -237,7 +248,7 @@ __global__ void __launch_bounds__(kQThreads, MODE == kModeSr ? 4 : 3)
     float v[16];
     unpack_raw16(cur, v);
     uint32_t sb;
-    const uint2 out = quantize_block<MODE>(v, 1.0f, g, rg, key, static_cast<uint32_t>(r * cols + cb * 16), &sb);
+    const uint2 out = quantize_block<MODE>(v, max_abs_raw16<T>(cur, v), 1.0f, g, rg, key, static_cast<uint32_t>(r * cols + cb * 16), &sb);
     __stcs(reinterpret_cast<uint2*>(codes + r * (cols / 2)) + cb, out);
     const int64_t sf_row = layout == BL_SF_ROWMAJOR ? r * cols16
                                                     : (r >> 7) * nc * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4;
@@ -398,34 +409,9 @@ __device__ __forceinline__ void load2(const T* p, float& a, float& b) {
 
 // v[j] = sum over i (ascending, every partial sum rounded to fp32: the reference's order) of p[i] * (-1)^popc(i & j),
 // p[i] = raw[i] * H[i][0], for H = diag(s) * Sylvester-Hadamard / 4. Outputs j and j' share every partial sum over
-// i < n when j = j' mod n, so the 16 sequential sums form a tree of 2 + 8 + 32 + 128 = 170 additions instead of 256.
-__device__ __forceinline__ void rotate16_tree(const float p[16], float v[16]) {
-  v[0] = p[0] + p[1];
-  v[1] = p[0] - p[1];
-#pragma unroll
-  for (int n = 2; n < 16; n <<= 1) {
-#pragma unroll
-    for (int j = 0; j < n; ++j) {
-      float a = v[j], b = v[j];
-#pragma unroll
-      for (int i = 0; i < n; ++i) {
-        if (__popc(i & j) & 1) {
-          a = a - p[n + i];
-          b = b + p[n + i];
-        } else {
-          a = a + p[n + i];
-          b = b - p[n + i];
-        }
-      }
-      v[j] = a;
-      v[n + j] = b;
-    }
-  }
-}
-
-// The same tree for two columns at once, one in each lane of packed fp32 pairs: half the instructions. (p holds
-// products by +-1/4, which are exact, so it does not matter that a packed product feeding a packed sum is contracted
-// into one fused multiply-add.)
+// i < n when j = j' mod n, so the 16 sequential sums form a tree of 2 + 8 + 32 + 128 = 170 additions instead of 256. Two
+// columns at once, one in each lane of packed fp32 pairs. (p holds products by +-1/4, which are exact, so it does not
+// matter that a packed product feeding a packed sum is contracted into one fused multiply-add.)
 __device__ __forceinline__ void rotate16_tree2(const f32x2 p[16], f32x2 v[16]) {
   v[0] = add2p(p[0], p[1]);
   v[1] = sub2p(p[0], p[1]);
@@ -447,17 +433,6 @@ __device__ __forceinline__ void rotate16_tree2(const f32x2 p[16], f32x2 v[16]) {
       v[j] = a;
       v[n + j] = b;
     }
-  }
-}
-
-// any 16 x 16 matrix: for each output the ascending sum over the inputs
-__device__ __forceinline__ void rotate16_generic(const float raw[16], const float* __restrict__ sH, float v[16]) {
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    float a = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) a = a + raw[i] * sH[i * 16 + j];
-    v[j] = a;
   }
 }
 
@@ -495,30 +470,56 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
     const float g = global_t(global, given);
     if (global_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) global_out[0] = g;
     const float rg = __frcp_rn(g);
-    float va[16], vb[16];
+    f32x2 v2[16];
     if (H == nullptr) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        va[i] = ra[i];
-        vb[i] = rb[i];
-      }
+      for (int i = 0; i < 16; ++i) v2[i] = pk(ra[i], rb[i]);
     } else if (structured) {
-      f32x2 p2[16], v2[16];
+      f32x2 p2[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) p2[i] = mul2p(pk(ra[i], rb[i]), pk(sH[i * 16], sH[i * 16]));
       rotate16_tree2(p2, v2);
+    } else {
+      // any other matrix: for each output the ascending sum over the inputs, which wait in local memory so that this
+      // route takes no registers from the usual one
+      float wait[32];
+      for (int i = 0; i < 16; ++i) {
+        wait[2 * i] = to_f<T>(p[i * K]);
+        wait[2 * i + 1] = to_f<T>(p[i * K + 1]);
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        float a = 0.0f, b = 0.0f;
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i) {
+          a = a + wait[2 * i] * sH[i * 16 + j];
+          b = b + wait[2 * i + 1] * sH[i * 16 + j];
+        }
+        v2[j] = pk(a, b);
+      }
+    }
+    float amax_a, amax_b;
+    {
+      float va[16], vb[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) upk(v2[i], va[i], vb[i]);
-    } else {
-      rotate16_generic(ra, sH, va);
-      rotate16_generic(rb, sH, vb);
+      amax_a = max_abs16(va);
+      amax_b = max_abs16(vb);
     }
-    uint32_t sb;
-    s_codes[2 * kp][mb] =
-        quantize_block<SR ? kModeSr : kModeRtn>(va, 1.0f, g, rg, key, static_cast<uint32_t>(static_cast<uint64_t>(k) * M + m), &sb);
-    s_scales[2 * kp][mb] = static_cast<uint8_t>(sb);
-    s_codes[2 * kp + 1][mb] =
-        quantize_block<SR ? kModeSr : kModeRtn>(vb, 1.0f, g, rg, key, static_cast<uint32_t>(static_cast<uint64_t>(k + 1) * M + m), &sb);
+    const uint32_t idx_a = static_cast<uint32_t>(static_cast<uint64_t>(k) * M + m), idx_b = idx_a + static_cast<uint32_t>(M);
+    const float fa = div_rn(amax_a, 6.0f, kInv6), fb = div_rn(amax_b, 6.0f, kInv6);
+    const uint32_t sa = e4m3_encode(div_rn(SR ? fa : fmaxf(fa, 1e-12f), g, rg));
+    const uint32_t sb = e4m3_encode(div_rn(SR ? fb : fmaxf(fb, 1e-12f), g, rg));
+    const float ta = e4m3_decode(sa) * g, tb = e4m3_decode(sb) * g;
+    uint32_t ca[2], cb[2];
+    if constexpr (SR)
+      e2m1_sr16x2(v2, ta > 0.0f ? __frcp_rn(ta) : 0.0f, tb > 0.0f ? __frcp_rn(tb) : 0.0f, idx_a * 0x27D4EB2Fu + key,
+                  idx_b * 0x27D4EB2Fu + key, ca, cb);
+    else
+      e2m1_rtn16x2(v2, ta, tb, rcp_approx(ta), rcp_approx(tb), ca, cb);
+    s_codes[2 * kp][mb] = make_uint2(ca[0], ca[1]);
+    s_codes[2 * kp + 1][mb] = make_uint2(cb[0], cb[1]);
+    s_scales[2 * kp][mb] = static_cast<uint8_t>(sa);
     s_scales[2 * kp + 1][mb] = static_cast<uint8_t>(sb);
   }
   __syncthreads();

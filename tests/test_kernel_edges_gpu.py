@@ -40,3 +40,36 @@ def test_requantize_t_ties_and_edges(N, K, g):
 def test_to_blocked_words_and_bytes(rows, cols16):
     s = np.random.default_rng(rows).integers(0, 256, (rows, cols16), dtype=np.uint8)
     assert np.array_equal(host(_ops.to_blocked(dev(s))), oracle.to_blocked(s).reshape(-1))
+
+
+def _sr_values(kind, shape, rng):
+    if kind == "normal":
+        return rng.standard_normal(shape).astype(np.float32)
+    if kind == "levels":                 # on levels, midpoints and just beside them: draws against fractions of 0, 1/2, ...
+        v = rng.choice(np.array([0, 0.25, 0.5, 0.75, 1, 1.25, 1.5, 2, 2.5, 3, 3.5, 4, 5, 6], np.float32), shape)
+        return v * rng.choice(np.array([1, -1, 1 + 2.0 ** -8, 2.0 ** -20, 2.0 ** -130], np.float32), shape)
+    return (rng.standard_normal(shape) * 10.0 ** rng.uniform(-30, 3, shape)).astype(np.float32)     # "wide"
+
+
+@pytest.mark.parametrize("kind", ["normal", "levels", "wide"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_stochastic_draws_on_all_bits(kind, dtype):
+    """Stochastic rounding of 2^22 elements, rows and transposed: about 60 of them draw a number whose upper 16 bits equal
+    those of their position between two levels and are decided on the bits below. Per-tensor scales above, at and below
+    the data's own (the last one saturates the block scales, so that values lie far beyond the last level)."""
+    rng = np.random.default_rng(7)
+    x = torch.from_numpy(_sr_values(kind, (2048, 2048), rng)).to(dtype)
+    xf = x.float().numpy()
+    g0 = np.float32(max(np.abs(xf).max() / 2688.0, 1e-12))
+    for g in (g0, np.float32(g0 * 4), np.float32(g0 / 37)):
+        rc, rs, _ = oracle.quantize_rows(xf, float(g), "sr", seed=11)
+        packed, sc = _ops.quantize_nvfp4(x.cuda(), dev(np.array([g], np.float32)), seed=11)
+        assert np.array_equal(host(packed), rc) and np.array_equal(host(sc), rs)
+    H = oracle.hadamard16()
+    for h in (H, None):
+        bound = np.float32(g0 * 4)
+        gt = oracle.global_from_bound(float(bound))
+        rc, rs = oracle.quantize_t(xf, h, gt, "sr", seed=5)
+        packed, sc, _ = _ops.quantize_nvfp4_t(x.cuda(), dev(h.astype(np.float32)) if h is not None else None, 5, 0,
+                                              dev(np.array([bound], np.float32)))
+        assert np.array_equal(host(packed), rc) and np.array_equal(host(sc), rs)
