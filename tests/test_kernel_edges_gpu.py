@@ -73,3 +73,26 @@ def test_stochastic_draws_on_all_bits(kind, dtype):
         packed, sc, _ = _ops.quantize_nvfp4_t(x.cuda(), dev(h.astype(np.float32)) if h is not None else None, 5, 0,
                                               dev(np.array([bound], np.float32)))
         assert np.array_equal(host(packed), rc) and np.array_equal(host(sc), rs)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_every_gate_value(dtype):
+    """Every 16-bit gate value (zeros of both signs, subnormals, infinities, NaN) through both kernels: the shared
+    reciprocal gives the bits of the expression with its two plain divisions. Laid out twice, so that in-range and
+    out-of-range values share vectors of eight in one and are alone in the other."""
+    bits = torch.arange(1 << 16, device="cuda", dtype=torch.int32)
+    order = torch.cat([bits, (bits * 40503) & 0xFFFF])
+    g = order.to(torch.int16).view(dtype)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    u = torch.randn(g.numel(), device="cuda", generator=gen).to(dtype)
+    da = torch.randn(g.numel(), device="cuda", generator=gen).to(dtype)
+    gf, uf, df = g.float(), u.float(), da.float()
+    d = 1.0 + torch.exp(-gf)
+    silu = (gf / d).to(dtype).float()
+    sig = 1.0 / d
+    want = ((silu * uf).to(dtype), ((df * uf).to(dtype).float() * sig * (1.0 + gf * (1.0 - sig))).to(dtype), (df * silu).to(dtype))
+    got = (_ops.swiglu_fwd(g, u), *_ops.swiglu_bwd(g, u, da))
+    for a, b in zip(got, want):
+        nan = b.isnan()
+        assert torch.equal(a.isnan(), nan)
+        assert torch.equal(a.view(torch.int16)[~nan], b.view(torch.int16)[~nan])
