@@ -677,25 +677,62 @@ __global__ void __launch_bounds__(kQThreads) requantize_t_kernel(const uint8_t* 
 
 // ------------------------------------------------------------------------------------------------ dequantize, layout
 
+// One thread expands 32 bytes of output at a time -- a block of 16 elements of a 16-bit type, half a block of fp32 --, the
+// next piece's codes and scale loaded first. Two levels come from one conversion to halves (exact; code 8, which reads as
+// +0, is cleared beforehand) instead of byte permutations and selects, and a
+// piece is one full-sector store: 12288 x 4096 to bf16 51 -> 27 us (4.9 TB/s), to fp32 53 -> 45 us.
 template <typename O>
 __global__ void __launch_bounds__(kQThreads) dequantize_kernel(const uint8_t* __restrict__ codes,
                                                                const uint8_t* __restrict__ scales,
-                                                               const float* __restrict__ global, int64_t nchunks,
+                                                               const float* __restrict__ global, int64_t pieces,
                                                                O* __restrict__ out) {
+  constexpr int kWords = sizeof(O) == 2 ? 2 : 1;               // 32-bit words of codes in a piece
+  const bool whole = (reinterpret_cast<uintptr_t>(out) & 31u) == 0;        // one store per piece: a full sector
   const float g = global[0];
-  for (int64_t ch = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; ch < nchunks;
-       ch += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint32_t word = reinterpret_cast<const uint32_t*>(codes)[ch];
-    const float s = e4m3_decode(scales[ch >> 1]) * g;
-    O o[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = from_f<O>(level_of_rank(rank_of_code((word >> (4 * i)) & 0xFu)) * s);
-    if constexpr (sizeof(O) == 4) {
-      reinterpret_cast<float4*>(out + ch * 8)[0] = *reinterpret_cast<float4*>(&o[0]);
-      reinterpret_cast<float4*>(out + ch * 8)[1] = *reinterpret_cast<float4*>(&o[4]);
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  auto load = [&](int64_t at, uint32_t w[kWords]) -> uint32_t {
+    if constexpr (kWords == 2) {
+      const uint2 v = reinterpret_cast<const uint2*>(codes)[at];
+      w[0] = v.x;
+      w[1] = v.y;
+      return scales[at];
     } else {
-      *reinterpret_cast<uint4*>(out + ch * 8) = *reinterpret_cast<uint4*>(&o[0]);
+      w[0] = reinterpret_cast<const uint32_t*>(codes)[at];
+      return scales[at >> 1];
     }
+  };
+  uint32_t w[kWords] = {}, sb = 0u;
+  if (i < pieces) sb = load(i, w);
+  while (i < pieces) {
+    const int64_t next = i + stride;
+    uint32_t wn[kWords] = {}, sn = 0u;
+    if (next < pieces) sn = load(next, wn);
+    const float s = e4m3_decode(sb) * g;
+    __align__(16) O o[8 * kWords];
+#pragma unroll
+    for (int h = 0; h < kWords; ++h) {
+      const uint32_t c = e2m1_drop_negative_zero(w[h]);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const float2 l = __half22float2(e2m1_levels2((c >> (8 * b)) & 0xFFu));
+        o[8 * h + 2 * b] = from_f<O>(l.x * s);
+        o[8 * h + 2 * b + 1] = from_f<O>(l.y * s);
+      }
+      w[h] = wn[h];
+    }
+    uint4* dst = reinterpret_cast<uint4*>(out + i * 8 * kWords);
+    const uint32_t* v = reinterpret_cast<const uint32_t*>(o);
+    if (whole) {
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                   "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                   : "memory");
+    } else {
+      dst[0] = reinterpret_cast<const uint4*>(o)[0];
+      dst[1] = reinterpret_cast<const uint4*>(o)[1];
+    }
+    sb = sn;
+    i = next;
   }
 }
 
@@ -971,14 +1008,14 @@ extern "C" int bl_nvfp4_dequantize(const uint8_t* codes, const uint8_t* scales, 
   BL_REQUIRE(aligned16(codes) && aligned16(out), "dequantize: codes and output must be 16-byte aligned");
   BL_DEVICE(device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int64_t nchunks = rows * cols / 8;
-  const int grid = grid_for(nchunks, kQThreads, device);
+  const int64_t pieces = rows * cols / (out_dtype == BL_F32 ? 8 : 16);
+  const int grid = grid_for(pieces, kQThreads, device);
   if (out_dtype == BL_BF16)
-    dequantize_kernel<<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, nchunks, static_cast<__nv_bfloat16*>(out));
+    dequantize_kernel<<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, pieces, static_cast<__nv_bfloat16*>(out));
   else if (out_dtype == BL_F16)
-    dequantize_kernel<<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, nchunks, static_cast<__half*>(out));
+    dequantize_kernel<<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, pieces, static_cast<__half*>(out));
   else
-    dequantize_kernel<<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, nchunks, static_cast<float*>(out));
+    dequantize_kernel<<<grid, kQThreads, 0, st>>>(codes, scales, global_scale, pieces, static_cast<float*>(out));
   BL_CUDA(cudaGetLastError());
   return 0;
 }

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import oracle
-from bitlattice_b200 import _ops
+from bitlattice_b200 import _C, _ops
 
 pytestmark = pytest.mark.gpu
 
@@ -96,3 +96,26 @@ def test_swiglu_every_gate_value(dtype):
         nan = b.isnan()
         assert torch.equal(a.isnan(), nan)
         assert torch.equal(a.view(torch.int16)[~nan], b.view(torch.int16)[~nan])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1, 16), (3, 48), (257, 32), (4096, 4096)])
+def test_dequantize_every_code(rows, cols, dtype):
+    """Level x (scale x global) rounded once to the output type, code 8 (-0) as +0, into an output that is 32-byte aligned
+    and into one that is only 16-byte aligned."""
+    rng = np.random.default_rng(rows + cols)
+    codes = rng.integers(0, 256, (rows, cols // 2), dtype=np.uint8)
+    scales = rng.integers(0, 0x7F, (rows, cols // 16), dtype=np.uint8)
+    g = torch.tensor([0.0137], device="cuda")
+    level = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6], device="cuda")
+    c = dev(codes).int()
+    nib = torch.stack([c & 15, c >> 4], -1).view(rows, cols)
+    s = dev(scales).view(torch.float8_e4m3fn).float() * g
+    want = (level[nib] * s.repeat_interleave(16, 1)).to(dtype)
+    raw = torch.zeros(rows * cols + 64, dtype=dtype, device="cuda")
+    shifted = raw[16 // raw.element_size():][:rows * cols].view(rows, cols)
+    packed, sc = dev(codes), dev(scales)
+    _C.call("bl_nvfp4_dequantize", packed.data_ptr(), sc.data_ptr(), g.data_ptr(), rows, cols,
+            shifted.data_ptr(), _C.DTYPE[dtype], 0, torch.cuda.current_stream().cuda_stream)
+    for got in (_ops.dequantize(packed, sc, g, None, "nvfp4", rows, cols, dtype), shifted):
+        assert torch.equal(got.contiguous().view(torch.uint8), want.view(torch.uint8))
