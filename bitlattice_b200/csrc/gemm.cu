@@ -433,6 +433,7 @@ struct GemmArgs {
   int64_t M, N, K, ldc;
   int out_dtype;
   int num_m, num_n;
+  int a_rows;              // tile kernel: rows of A a stage loads (all 128, or the few of a single ragged tile)
   int accumulate;          // 1: out += result, the sum rounded as a dense add of two tensors of the output type
 };
 
@@ -512,9 +513,15 @@ __device__ __forceinline__ void store_row32(O* dst, const uint32_t acc[32], floa
   else store_row32_impl<O, false>(dst, acc, alpha, ncols_valid);
 }
 
+// One 128 x 128 tile per CTA, for problems with fewer tiles than SMs. What bounds it is the latency of a k-tile (256 of K)
+// times their number, so six stages are in flight and both role warps run converged, one elected lane issuing (with a
+// single lane running on its own every tcgen05 and copy instruction cost some 90 issue cycles, 0.75 us per k-tile). Device
+// times with L2 flushed, an empty problem taking 8 us: 16 x 4096 x 12288 41 -> 25 us, 16 x 1024 x 4096 18 -> 13 us,
+// 16 x 12288 x 4096 20 -> 15 us, 256 x 4096 x 4096 20 -> 14 us. (Tiles 64 wide on twice the CTAs: 23, 12, 21 and 14 us.)
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                                                             const __grid_constant__ CUtensorMap map_b, GemmArgs args) {
+  static_assert(BN == 128, "a tile reads one 128-row block of B scales");
   using S = GemmSmem<BN, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -544,11 +551,10 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constan
 
   const int num_k_tiles = static_cast<int>((args.K + kBK - 1) / kBK);
   const int nkb = static_cast<int>((args.K + 63) / 64);               // scale blobs per 128 rows along K
-  const int nrb_b = static_cast<int>((args.N + 127) / 128);           // 128-row scale blocks of B
 
-  constexpr uint32_t kTmemCols = BN <= 64 ? 128 : (BN <= 192 ? 256 : 512);
+  constexpr uint32_t kTmemCols = 256;
   constexpr uint32_t kSfaCol = BN;            // accumulator: columns [0, BN); then 16 columns of A scales
-  constexpr uint32_t kSfbCol = BN + 16;       // then (BN/32)*4 columns of B scales
+  constexpr uint32_t kSfbCol = BN + 16;       // then 16 columns of B scales
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -567,57 +573,64 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- producer
+    // ---------------------------------------------------------------- producer: whole warp converged, one lane issues
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_b)) : "memory");
-      for (int kt = 0; kt < num_k_tiles; ++kt) {
-        const int s = kt % STAGES;
-        const uint32_t round = kt / STAGES;
-        if (round > 0 && !mbar_wait(empty_bar(s), (round - 1) & 1, abort_flag, 1)) break;
-        const uint32_t stage = base + s * S::kStage;
-        const int blobs = min(4, nkb - kt * 4);
-        const uint32_t sf_bytes = blobs * 512u;
-        const int b_blocks = min(BN / 128, nrb_b - tile_n * (BN / 128));     // 128-row scale blocks of B that exist
-        mbar_expect_tx(full_bar(s), S::kA + S::kB + sf_bytes * (1 + b_blocks));
-        tma_load_2d(stage, &map_a, kt * (kBK / 2), static_cast<int>(m0), full_bar(s));
-        tma_load_2d(stage + S::kA, &map_b, kt * (kBK / 2), static_cast<int>(n0), full_bar(s));
-        const uint8_t* sfa = args.a_sf + (static_cast<int64_t>(tile_m) * nkb + kt * 4) * 512;
-        bulk_load(stage + S::kA + S::kB, sfa, sf_bytes, full_bar(s));
-#pragma unroll
-        for (int h = 0; h < b_blocks; ++h) {
-          const uint8_t* sfb = args.b_sf + ((static_cast<int64_t>(tile_n) * (BN / 128) + h) * nkb + kt * 4) * 512;
-          bulk_load(stage + S::kA + S::kB + S::kSFA + h * 2048, sfb, sf_bytes, full_bar(s));
-        }
+    }
+    __syncwarp();
+    const uint8_t* sfa = args.a_sf + static_cast<int64_t>(tile_m) * nkb * 512;
+    const uint8_t* sfb = args.b_sf + static_cast<int64_t>(tile_n) * nkb * 512;
+    int s = 0;
+    uint32_t phase = 1;                                    // parity that means "stage is free" (free at the start)
+    for (int kt = 0; kt < num_k_tiles; ++kt) {
+      if (!__all_sync(0xffffffffu, mbar_wait(empty_bar(s), phase, abort_flag, 1))) break;
+      const uint32_t q = elect_one();
+      const uint32_t stage = base + s * S::kStage;
+      const uint32_t sf_bytes = min(4, nkb - kt * 4) * 512u;
+      mbar_expect_tx_if(q, full_bar(s), args.a_rows * (kBK / 2) + S::kB + 2 * sf_bytes);
+      tma_load_2d_if(q, stage + S::kA, &map_b, kt * (kBK / 2), static_cast<int>(n0), full_bar(s));
+      tma_load_2d_if(q, stage, &map_a, kt * (kBK / 2), static_cast<int>(m0), full_bar(s));
+      bulk_load_if(q, stage + S::kA + S::kB, sfa + kt * 2048, sf_bytes, full_bar(s));
+      bulk_load_if(q, stage + S::kA + S::kB + S::kSFA, sfb + kt * 2048, sf_bytes, full_bar(s));
+      if (++s == STAGES) {
+        s = 0;
+        phase ^= 1;
       }
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      // instruction descriptor: E2M1 x E2M1, UE4M3 scales, K-major A and B, N = BN, M = 128, dense K = 64
-      constexpr uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) | (8u << 24);
-      bool ok = true;
-      for (int kt = 0; kt < num_k_tiles && ok; ++kt) {
-        const int s = kt % STAGES;
-        ok = mbar_wait(full_bar(s), (kt / STAGES) & 1, abort_flag, 2);
-        if (!ok) break;
-        tcgen05_fence_after();
-        const uint32_t stage = base + s * S::kStage;
-        const int blocks = min(4, nkb - kt * 4);
+    // ---------------------------------------------------------------- MMA issue: whole warp converged, one lane issues
+    // instruction descriptor: E2M1 x E2M1, UE4M3 scales, K-major A and B, N = BN, M = 128, dense K = 64
+    constexpr uint32_t idesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) | (8u << 24);
+    int s = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int kt = 0; kt < num_k_tiles; ++kt) {
+      ok = __all_sync(0xffffffffu, mbar_wait(full_bar(s), phase, abort_flag, 2));
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint32_t q = elect_one();
+      const uint32_t stage = base + s * S::kStage;
+      const int blocks = min(4, nkb - kt * 4);
+      const uint64_t adesc = operand_desc(stage), bdesc = operand_desc(stage + S::kA);
+      const uint64_t sdesc = scale_desc(stage + S::kA + S::kB);
+      if (blocks == 4) {
+        issue_k_tile<1, 0, 1>(q, tmem_base, tmem_base + kSfaCol, tmem_base + kSfbCol, sdesc, adesc, bdesc, idesc, kt != 0);
+      } else {
         for (int j = 0; j < blocks; ++j) {
-          tmem_copy_scales(tmem_base + kSfaCol + 4 * j, scale_desc(stage + S::kA + S::kB + j * 512));
-#pragma unroll
-          for (int h = 0; h < BN / 128; ++h)
-            tmem_copy_scales(tmem_base + kSfbCol + (BN / 32) * j + 4 * h,
-                             scale_desc(stage + S::kA + S::kB + S::kSFA + h * 2048 + j * 512));
+          tmem_copy_scales_if<1>(q, tmem_base + kSfaCol + 4 * j, sdesc + 32u * j);
+          tmem_copy_scales_if<1>(q, tmem_base + kSfbCol + 4 * j, sdesc + 128u + 32u * j);
         }
-        const uint64_t adesc = operand_desc(stage), bdesc = operand_desc(stage + S::kA);
         for (int j = 0; j < blocks; ++j)
-          mma_nvf4(tmem_base, adesc + 2u * j, bdesc + 2u * j, idesc, tmem_base + kSfaCol + 4 * j,
-                   tmem_base + kSfbCol + (BN / 32) * j, (kt | j) != 0);
-        mma_commit(empty_bar(s));
+          mma_nvf4_if<1>(q, tmem_base, adesc + 2u * j, bdesc + 2u * j, idesc, tmem_base + kSfaCol + 4 * j,
+                         tmem_base + kSfbCol + 4 * j, (kt | j) != 0);
       }
-      if (ok) mma_commit(acc_bar);
+      mma_commit_if<1>(q, empty_bar(s));
+      if (kt == num_k_tiles - 1) mma_commit_if<1>(q, acc_bar);
+      if (++s == STAGES) {
+        s = 0;
+        phase ^= 1;
+      }
     }
   } else {
     // ---------------------------------------------------------------- epilogue
@@ -1360,7 +1373,10 @@ template <int BN, int STAGES>
 static int launch_gemm(const uint8_t* a_codes, const uint8_t* b_codes, GemmArgs args, cudaStream_t st) {
   using S = GemmSmem<BN, STAGES>;
   CUtensorMap map_a, map_b;
-  if (int rc = make_operand_map(&map_a, a_codes, args.M, args.K, kBM)) return rc;
+  // A few rows (decode): only those are loaded. The rest of the A tile keeps what the memory held before; it reaches only
+  // accumulator rows that are not stored.
+  args.a_rows = args.M <= kBM / 2 ? static_cast<int>((args.M + 7) / 8) * 8 : kBM;
+  if (int rc = make_operand_map(&map_a, a_codes, args.M, args.K, args.a_rows)) return rc;
   if (int rc = make_operand_map(&map_b, b_codes, args.N, args.K, BN)) return rc;
   args.num_m = static_cast<int>((args.M + kBM - 1) / kBM);
   args.num_n = static_cast<int>((args.N + BN - 1) / BN);
@@ -1472,7 +1488,7 @@ static int gemm_entry(const uint8_t* a_codes, const uint8_t* a_sf, const float* 
   args.K = K;
   args.ldc = ldc;
   args.out_dtype = out_dtype;
-  args.num_m = args.num_n = 0;
+  args.num_m = args.num_n = args.a_rows = 0;
   args.accumulate = accumulate ? 1 : 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int kernel = g_kernel_choice.load(std::memory_order_relaxed);
@@ -1489,7 +1505,7 @@ static int gemm_entry(const uint8_t* a_codes, const uint8_t* a_sf, const float* 
   }
   if (kernel == BL_GEMM_PAIR) return launch_pair<256, 5>(a_codes, b_codes, args, device, st);
   if (kernel == BL_GEMM_PERSISTENT) return launch_persistent<4, 0>(a_codes, b_codes, args, device, st);
-  return launch_gemm<128, 3>(a_codes, b_codes, args, st);
+  return launch_gemm<128, 6>(a_codes, b_codes, args, st);
 }
 
 extern "C" int bl_nvfp4_gemm(const uint8_t* a_codes, const uint8_t* a_sf, const float* a_global, const uint8_t* b_codes,

@@ -119,3 +119,22 @@ def test_dequantize_every_code(rows, cols, dtype):
             shifted.data_ptr(), _C.DTYPE[dtype], 0, torch.cuda.current_stream().cuda_stream)
     for got in (_ops.dequantize(packed, sc, g, None, "nvfp4", rows, cols, dtype), shifted):
         assert torch.equal(got.contiguous().view(torch.uint8), want.view(torch.uint8))
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 64, 65, 129])
+@pytest.mark.parametrize("N,K", [(8, 32), (136, 288), (384, 1792), (1000, 4128)])
+def test_tile_gemm_few_rows(M, N, K):
+    """The tile kernel where it loads only the rows of A that exist (M <= 64) and where it loads whole tiles, k-tiles cut
+    off after 1, 2 and 4 blocks and more k-tiles than stages, against the persistent kernel bit for bit."""
+    gen = torch.Generator(device="cuda").manual_seed(M * N + K)
+    a, b = (torch.randn(r, K, device="cuda", generator=gen).to(torch.bfloat16) for r in (M, N))
+    qa, qb = (_ops.amax_quantize_nvfp4(t, -1, 0, blocked=True) for t in (a, b))
+    outs = []
+    try:
+        for kernel in ("tile", "persistent"):
+            _ops.gemm_select(kernel)
+            outs.append(_ops.nvfp4_gemm(qa[0], qa[1], qa[2][1:2], qb[0], qb[1], qb[2][1:2]))
+    finally:
+        _ops.gemm_select("auto")
+    assert torch.equal(outs[0], outs[1]) and outs[0].isfinite().all()
+    assert _ops.gemm_status(0) == 0
