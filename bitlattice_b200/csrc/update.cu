@@ -250,6 +250,7 @@ struct StepParams {
   float r_lo, r_hi;  // exp(-kappa), exp(+kappa)
   int mode;          // BL_ROUND_*
   float strat_k;
+  int rows_per_thread;
 };
 
 // ---- per-thread work unit: one scale group of 16 consecutive elements ------------------------------------------------
@@ -348,6 +349,59 @@ __device__ __forceinline__ void build_tables(float2* lutAL, float4* plut, int pb
     if (plut24) plut24[tid] = make_float4(w, su * 16777216.0f, sd * 16777216.0f,
                                           __uint_as_float(code_of_rank(min(rk + 1, 14))));
   }
+}
+
+// The (level, latent) table of build_tables once per lane: entry e of lane l at e * 256 + 4 l (level) and + 128 (latent), so
+// that the 32 random look-ups of a warp touch 32 different banks, a byte permutation forms the offset (entry in byte 1, lane
+// in byte 0) and the two values arrive in registers of their own. 8, 16 or 64 KB for 1-, 2- and 4-bit containers.
+template <int PCB> constexpr int kLaneTableBytes = (16 << PCB) * 256;
+
+template <int PCB>
+__device__ __forceinline__ void build_lane_table(unsigned char* tab, const float2* lutAL, int tid) {
+  constexpr int kEntries = 16 << PCB, kParts = kThreads / kEntries;
+  static_assert(kEntries * kParts == kThreads && 32 % kParts == 0, "every thread fills part of one entry");
+  const float2 al = lutAL[tid % kEntries];
+  unsigned char* entry = tab + (tid % kEntries) * 256;
+#pragma unroll 8
+  for (int j = 0; j < 32 / kParts; ++j) {
+    const int l = (tid + (tid / kEntries) * (32 / kParts) + j) & 31;        // lanes of a warp start at different banks
+    reinterpret_cast<float*>(entry)[l] = al.x;
+    reinterpret_cast<float*>(entry)[32 + l] = al.y;
+  }
+}
+
+// Index bytes code | phase << 4 of the eight elements of half a group: element 2 k in byte k of ev, 2 k + 1 in byte k of od.
+template <int PCB>
+__device__ __forceinline__ void index_bytes(uint32_t codes, uint32_t phase, uint32_t& ev, uint32_t& od) {
+  uint32_t pe, po;                              // phases of the even / odd elements, shifted to bit 4 of their bytes
+  if constexpr (PCB == 4) {
+    pe = (phase << 4) & 0xF0F0F0F0u;
+    po = phase & 0xF0F0F0F0u;
+  } else if constexpr (PCB == 2) {              // phase: 16 bits
+    uint32_t x = __byte_perm(phase, 0u, 0x4140u);
+    x = (x | (x << 4)) & 0x0F0F0F0Fu;           // two elements per byte
+    pe = (x << 4) & 0x30303030u;
+    po = (x << 2) & 0x30303030u;
+  } else {                                      // phase: 8 bits; the product moves bit 2 k to bit 8 k + 4
+    pe = ((phase & 0x55u) * 0x00410410u) & 0x10101010u;
+    po = (((phase >> 1) & 0x55u) * 0x00410410u) & 0x10101010u;
+  }
+  ev = (codes & 0x0F0F0F0Fu) | pe;
+  od = ((codes >> 4) & 0x0F0F0F0Fu) | po;
+}
+
+// The containers of eight elements, element 2 k in byte k of pe, 2 k + 1 in byte k of po (values below 1 << PCB).
+template <int PCB>
+__device__ __forceinline__ uint32_t join_phases(uint32_t pe, uint32_t po) {
+  uint32_t w = pe | (po << PCB);
+  if constexpr (PCB == 2) {
+    w = (w | (w >> 4)) & 0x00FF00FFu;
+    w = __byte_perm(w, 0u, 0x4420u);
+  } else if constexpr (PCB == 1) {
+    w = w | (w >> 6);
+    w = (w & 0x0Fu) | ((w >> 12) & 0xF0u);
+  }
+  return w;
 }
 
 __device__ __forceinline__ float draw_u(int mode, uint32_t idx, uint32_t key, float strat_j, float strat_k) {
@@ -504,7 +558,105 @@ __device__ __forceinline__ uint32_t sum_sq4(uint32_t codes) {
   return __dp4a(lo, 0x01010101u, __dp4a(hi, 0x01010101u, 0u));
 }
 
-constexpr int kRowsPerThread = 8;     // rows a thread of the update kernel walks at most
+// true when every |v[i]| lies in [lo, hi] (a NaN gives false): three-input minima and maxima, one instruction per element
+__device__ __forceinline__ bool in_range16(const float v[16], float lo, float hi) {
+  float mn = v[15], mx = v[15];
+#pragma unroll
+  for (int i = 0; i < 14; i += 2) {
+    asm("min.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(mn) : "f"(v[i]), "f"(v[i + 1]));
+    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(v[i]), "f"(v[i + 1]));
+  }
+  asm("min.NaN.abs.f32 %0, %0, %1, %1;" : "+f"(mn) : "f"(v[14]));
+  asm("max.NaN.abs.f32 %0, %0, %1, %1;" : "+f"(mx) : "f"(v[14]));
+  return mn >= lo && mx <= hi;
+}
+
+// ---- projection with at most 4 phase bits
+// E2M1 is a float with one mantissa bit and subnormals below 1, so the bit pattern of |t| * 2^-126 is the position of |t| on
+// the lattice counted in levels, times 2^22 (truncated, where |t| < 1): a level every 2^22, linear between them, which is
+// what the phase coordinate counts too, 2^pb steps to a level. Times 2^(2 + pb) the number of whole steps K is in the top
+// byte and the fraction, as a multiple of 2^-24, below it. The draw n = hash >> 8 of a positive t rounds up iff
+// n * 2^-24 < fraction: the carry of adding 2^24 - 1 - n. For a negative t rounding down the value is rounding up the
+// magnitude, iff fraction >= 1 - n * 2^-24: the carry of adding n. So one product and one sum per element give K after
+// rounding; level and phase of four elements are then split in the bytes of one register (split_levels). z collects the
+// largest fraction sum: within 2^(2 + pb) + 1 <= 65 of the carry the truncated bits could matter, and the group takes the
+// general route (66 of 2^24 sums).
+//
+// What bounds the loop is the issue of instructions and their latency (16 warps on an SM, no pipe above 53 %): 66 per element
+// against 83 when the projection found the nearest level by conversion, looked up 16 bytes by code and selected by side and
+// carry (shared-memory wavefronts 60 % then, 25 % now). With the lane tables and the prefetched rows: three decoder layers
+// (578.7 M weights, colnorm, 4 bits) 1960 -> 1455 us, 12288 x 4096 sign 155 -> 131 us, fp32 sign 2 bits 160 -> 135 us.
+static __device__ __constant__ uint32_t kUpdateMul[1] = {256u};   // from constant memory, so that the product stays a product
+constexpr uint32_t kUndecided = 0u - (66u << 8);
+
+// ---- the next row of a thread
+// A thread's codes, phases and gradients of the next row are copied into its own slots of shared memory while it works on
+// the current row: the loop has no registers left to hold them (128 with the column denominators of colnorm), and without
+// them every row began with a wait for memory that the 16 warps of an SM did not cover (a fifth of all cycles). Slots of one
+// stage: 16-byte pieces of the gradient, then 8 bytes of codes, then the phases, each [kThreads] wide. A thread reads only
+// what it copied itself, so there is nothing to synchronise but its own copies.
+template <int PCB, typename GT>
+struct RowSlots {
+  static constexpr int kGrad = sizeof(GT);                                  // 16-byte pieces of 16 gradients
+  static constexpr int kPhase = PCB >= 2 ? 2 * PCB : 0;                     // bytes (the 2 of 1-bit containers go by register)
+  static constexpr int kStage = kThreads * (16 * kGrad + 8 + kPhase);
+  static constexpr int kTotal = 2 * kStage;
+};
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(unsigned char* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "n"(BYTES)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_close() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_async_wait_all_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+template <int PCB, typename GT>
+__device__ __forceinline__ void fetch_row(unsigned char* stage, const TensorDesc& T, const GT* grad, int64_t r, int64_t cg, int64_t cols) {
+  using R = RowSlots<PCB, GT>;
+#pragma unroll
+  for (int i = 0; i < R::kGrad; ++i)
+    copy_async<16>(stage + (i * kThreads + threadIdx.x) * 16, reinterpret_cast<const unsigned char*>(grad + r * cols + cg * 16) + 16 * i);
+  unsigned char* at = stage + R::kGrad * kThreads * 16;
+  copy_async<8>(at + threadIdx.x * 8, T.codes + r * (cols / 2) + cg * 8);
+  if constexpr (R::kPhase != 0)
+    copy_async<R::kPhase>(at + kThreads * 8 + threadIdx.x * R::kPhase, T.phase + r * (cols * PCB / 8) + cg * (2 * PCB));
+}
+
+__device__ __forceinline__ void project_pair(float t0, float t1, uint32_t h0, uint32_t h1, uint32_t spread, uint32_t byte256,
+                                             uint32_t& S0, uint32_t& S1, uint32_t& z) {
+  constexpr float kDown = 1.1754943508222875e-38f;                                   // 2^-126
+  float b0, b1;
+  upk(mul2p_down(pk(fminf(fabsf(t0), 6.0f), fminf(fabsf(t1), 6.0f)), pk(kDown, kDown)), b0, b1);
+  const uint32_t m0 = static_cast<uint32_t>(static_cast<int32_t>(__float_as_uint(t0)) >> 31);
+  const uint32_t m1 = static_cast<uint32_t>(static_cast<int32_t>(__float_as_uint(t1)) >> 31);
+  h0 = (h0 ^ (h0 >> 16)) * 0x7FEB352Du;
+  h1 = (h1 ^ (h1 >> 16)) * 0x7FEB352Du;
+  h0 = (h0 ^ (h0 >> 15)) * 0x846CA68Bu;
+  h1 = (h1 ^ (h1 >> 15)) * 0x846CA68Bu;
+  S0 = __float_as_uint(b0) * spread + (~(h0 ^ (h0 >> 16) ^ m0) >> 8);
+  S1 = __float_as_uint(b1) * spread + (~(h1 ^ (h1 >> 16) ^ m1) >> 8);
+  z = __vimax3_u32(z, S0 * byte256, S1 * byte256);
+}
+
+// {sign of a, sign of b} as bytes 0x00 / 0xFF in the lower half (the intrinsic masks off the selector bit that replicates signs)
+__device__ __forceinline__ uint32_t top_signs(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, 0x00FB;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
+// Steps K (top bytes of S) and signs (top bits of sg) of four elements -> code nibbles and phase bits, element k in byte k.
+// The signed count +-K is level * 2^pb + phase with the phase in [-half, half): level magnitude (K + half) >> pb, one less in
+// the numerator for negative values, phase = the low bits of the signed count. No byte carries into the next: K <= 7 * 2^pb.
+__device__ __forceinline__ void split_levels(const uint32_t S[4], const uint32_t sg[4], int pb, uint32_t half4, uint32_t pmask4,
+                                             uint32_t& code, uint32_t& phase) {
+  const uint32_t K = __byte_perm(__byte_perm(S[0], S[1], 0x0073u), __byte_perm(S[2], S[3], 0x0073u), 0x5410u);
+  const uint32_t m = __byte_perm(top_signs(sg[0], sg[1]), top_signs(sg[2], sg[3]), 0x5410u);
+  const uint32_t one = m & 0x01010101u;
+  phase = (((K ^ m) & pmask4) + one) & pmask4;
+  code = (((K - one + half4) >> pb) & 0x07070707u) | (m & 0x08080808u);
+}
 
 __host__ __device__ inline int update_bx(int cols) {
   const int cpr = cols / 16;
@@ -512,11 +664,14 @@ __host__ __device__ inline int update_bx(int cols) {
   while (bx < kThreads && bx < cpr) bx <<= 1;
   return bx;
 }
-__host__ __device__ inline int update_blocks(int rows, int cols) {
+__host__ __device__ inline int update_row_blocks(int rows, int by, int rows_per_thread) {
+  const int64_t per = static_cast<int64_t>(by) * rows_per_thread;
+  return static_cast<int>((rows + per - 1) / per);
+}
+__host__ __device__ inline int update_blocks(int rows, int cols, int rows_per_thread) {
   const int bx = update_bx(cols), by = kThreads / bx;
   const int gx = (cols / 16 + bx - 1) / bx;
-  const int gy = (rows + by * kRowsPerThread - 1) / (by * kRowsPerThread);
-  return gx * gy;
+  return gx * update_row_blocks(rows, by, rows_per_thread);
 }
 
 // FAST: stochastic rounding with 1..7 phase bits. Its arithmetic runs on packed pairs (element i with element i + 8,
@@ -533,16 +688,22 @@ template <int PCB, int DIR, typename GT, bool FAST>
 __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_constant__ Batch B, unsigned char* __restrict__ scratch, int has_stats,
                                                             StepParams P) {
   using PW = typename PhaseWord<PCB>::type;
+  constexpr bool kNarrow = FAST && PCB <= 4;                // at most 4 phase bits: see project_pair
+  extern __shared__ __align__(256) unsigned char lane_table[];
   __shared__ float2 lutAL[16 << PCB];                       // (level, latent) pairs: one load per element
   __shared__ float4 plut[16];
-  __shared__ float4 plut24[FAST ? 16 : 1];
-  build_tables<PCB>(lutAL, plut, P.pb, threadIdx.x, FAST ? plut24 : nullptr);
+  __shared__ float4 plut24[FAST && !kNarrow ? 16 : 1];
+  build_tables<PCB>(lutAL, plut, P.pb, threadIdx.x, FAST && !kNarrow ? plut24 : nullptr);
   __syncthreads();
+  if constexpr (kNarrow) {
+    build_lane_table<PCB>(lane_table, lutAL, threadIdx.x);
+    __syncthreads();
+  }
 
   int ti = 0;
   int blk = blockIdx.x;
   for (;; ++ti) {
-    const int n = update_blocks(B.t[ti].rows, B.t[ti].cols);
+    const int n = update_blocks(B.t[ti].rows, B.t[ti].cols, P.rows_per_thread);
     if (blk < n || ti == B.count - 1) break;
     blk -= n;
   }
@@ -550,7 +711,7 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
   const int64_t rows = T.rows, cols = T.cols;
   const int bx = update_bx(T.cols), by = kThreads / bx;
   const int gx = (T.cols / 16 + bx - 1) / bx;
-  const int gy = (T.rows + by * kRowsPerThread - 1) / (by * kRowsPerThread);
+  const int gy = update_row_blocks(T.rows, by, P.rows_per_thread);
   const int tx = threadIdx.x & (bx - 1), ty = threadIdx.x / bx;
   const int64_t cg = static_cast<int64_t>(blk % gx) * bx + tx;      // 16-column group of this thread
   if (cg * 16 >= cols) return;
@@ -574,12 +735,15 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
     const float rgs = __frcp_rn(gs);
     const GT* grad = static_cast<const GT*>(T.grad);
     const int64_t code_stride = cols / 2, phase_stride = cols * PCB / 8, scale_stride = cols / 16;
-    const uint32_t pmask = (1u << P.pb) - 1u;
-    const int half_i = 1 << (P.pb - 1);
+    [[maybe_unused]] const uint32_t pmask = (1u << P.pb) - 1u;
+    [[maybe_unused]] const int half_i = 1 << (P.pb - 1);
+    [[maybe_unused]] const uint32_t half4 = static_cast<uint32_t>(half_i) * 0x01010101u, pmask4 = pmask * 0x01010101u;
     const bool fit = P.rule != BL_RULE_FIXED, latent = P.rule == BL_RULE_FIT_LATENT;
     const bool decay_one = P.decay == 1.0f;                   // no weight decay: the products by it are exact copies
     const f32x2 ndiv2 = pk(-div, -div), rdiv2 = pk(__frcp_rn(div), __frcp_rn(div));
     const f32x2 nlr2 = pk(-P.lr, -P.lr), decay2 = pk(P.decay, P.decay);
+    [[maybe_unused]] const uint32_t lane4 = (threadIdx.x & 31u) * 4u;
+    [[maybe_unused]] const uint32_t spread = 1u << (2 + P.pb), byte256 = kUpdateMul[0];
 
     // column denominators of the thread's group as pairs (i, i + 8), and the range bounds that depend on them
     f32x2 nden2[DIR == 3 ? 8 : 1], rden2[DIR == 3 ? 8 : 1];
@@ -605,14 +769,53 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
     const float hi_c = dmin * 3.1691265e29f;                                         // 2^98 (may overflow to +inf: no bound)
     const float hi_w = dmin * div * 1.1529215e18f;                                   // 2^60
 
+    [[maybe_unused]] unsigned char* slots = lane_table + (kNarrow ? kLaneTableBytes<PCB> : 0);
+    [[maybe_unused]] int stage = 0;
+    uint32_t sb_next = 0u;
+    [[maybe_unused]] PW pw_next{};
+    if constexpr (kNarrow) {
+      if (row_first < rows) {
+        fetch_row<PCB>(slots, T, grad, row_first, cg, cols);
+        sb_next = T.scales_in[row_first * scale_stride + cg];
+        if constexpr (PCB == 1) pw_next = *reinterpret_cast<const PW*>(T.phase + row_first * phase_stride + cg * 2);
+      }
+      copy_async_close();
+    }
     for (int64_t r = row_first; r < rows; r += row_step) {
       // ---- loads
-      const uint2 cw = *reinterpret_cast<const uint2*>(T.codes + r * code_stride + cg * 8);
-      const PW pw = *reinterpret_cast<const PW*>(T.phase + r * phase_stride + cg * (2 * PCB));
+      uint2 cw;
+      PW pw;
       float gv[16];
-      load8(grad + r * cols + cg * 16, gv);
-      load8(grad + r * cols + cg * 16 + 8, gv + 8);
-      const uint32_t sb_old = T.scales_in[r * scale_stride + cg];
+      uint32_t sb_old;
+      if constexpr (kNarrow) {
+        using R = RowSlots<PCB, GT>;
+        sb_old = sb_next;
+        pw = pw_next;
+        const unsigned char* cur = slots + stage * R::kStage;
+        stage ^= 1;
+        if (r + row_step < rows) {
+          fetch_row<PCB>(slots + stage * R::kStage, T, grad, r + row_step, cg, cols);
+          sb_next = T.scales_in[(r + row_step) * scale_stride + cg];
+          if constexpr (PCB == 1) pw_next = *reinterpret_cast<const PW*>(T.phase + (r + row_step) * phase_stride + cg * 2);
+        }
+        copy_async_close();
+        copy_async_wait_all_but_last();
+        __align__(16) GT raw[16];
+#pragma unroll
+        for (int i = 0; i < R::kGrad; ++i)
+          reinterpret_cast<uint4*>(raw)[i] = *reinterpret_cast<const uint4*>(cur + (i * kThreads + threadIdx.x) * 16);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) gv[i] = to_f<GT>(raw[i]);
+        cur += R::kGrad * kThreads * 16;
+        cw = *reinterpret_cast<const uint2*>(cur + threadIdx.x * 8);
+        if constexpr (R::kPhase != 0) pw = *reinterpret_cast<const PW*>(cur + kThreads * 8 + threadIdx.x * R::kPhase);
+      } else {
+        cw = *reinterpret_cast<const uint2*>(T.codes + r * code_stride + cg * 8);
+        pw = *reinterpret_cast<const PW*>(T.phase + r * phase_stride + cg * (2 * PCB));
+        load8(grad + r * cols + cg * 16, gv);
+        load8(grad + r * cols + cg * 16 + 8, gv + 8);
+        sb_old = T.scales_in[r * scale_stride + cg];
+      }
       const float s_old = e4m3_decode(sb_old) * gs;
       const float inv_s = __frcp_rn(s_old);
       const f32x2 sold2 = pk(s_old, s_old), nsold2 = pk(-s_old, -s_old), rsold2 = pk(inv_s, inv_s);
@@ -632,28 +835,33 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
       // ---- latent target and the sums of the scale fit
       f32x2 tau2[8];
       f32x2 sat2 = pk(0.0f, 0.0f), stt2 = pk(0.0f, 0.0f);
-      // table indices (code | phase << 4). With 4-bit containers the nibbles of a code word and of a phase word are
-      // interleaved into index bytes four at a time: even elements (c & 0x0F0F0F0F) | ((p << 4) & 0xF0F0F0F0), odd
-      // elements ((c >> 4) & 0x0F0F0F0F) | (p & 0xF0F0F0F0); an index is then one byte extraction.
       [[maybe_unused]] uint32_t ev[2], od[2];
-      if constexpr (PCB == 4) {
-        ev[0] = (cw.x & 0x0F0F0F0Fu) | ((pw.x << 4) & 0xF0F0F0F0u);
-        od[0] = ((cw.x >> 4) & 0x0F0F0F0Fu) | (pw.x & 0xF0F0F0F0u);
-        ev[1] = (cw.y & 0x0F0F0F0Fu) | ((pw.y << 4) & 0xF0F0F0F0u);
-        od[1] = ((cw.y >> 4) & 0x0F0F0F0Fu) | (pw.y & 0xF0F0F0F0u);
+      if constexpr (kNarrow) {
+        if constexpr (PCB == 4) {
+          index_bytes<4>(cw.x, pw.x, ev[0], od[0]);
+          index_bytes<4>(cw.y, pw.y, ev[1], od[1]);
+        } else {
+          index_bytes<PCB>(cw.x, pw & ((1u << (8 * PCB)) - 1u), ev[0], od[0]);
+          index_bytes<PCB>(cw.y, pw >> (8 * PCB), ev[1], od[1]);
+        }
       }
+      if constexpr (DIR != 2) ok = ok && in_range16(gv, g_lo, g_hi);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        uint32_t ia, ib;
-        if constexpr (PCB == 4) {
-          ia = __byte_perm((i & 1) ? od[0] : ev[0], 0u, 0x4440u | static_cast<uint32_t>(i >> 1));
-          ib = __byte_perm((i & 1) ? od[1] : ev[1], 0u, 0x4440u | static_cast<uint32_t>(i >> 1));
+        float a0, a1, l0, l1;
+        if constexpr (kNarrow) {
+          const uint32_t sel = 0x5504u | (static_cast<uint32_t>(i >> 1) << 4);
+          const uint32_t oa = __byte_perm((i & 1) ? od[0] : ev[0], lane4, sel);
+          const uint32_t ob = __byte_perm((i & 1) ? od[1] : ev[1], lane4, sel);
+          a0 = *reinterpret_cast<const float*>(lane_table + oa);
+          l0 = *reinterpret_cast<const float*>(lane_table + oa + 128);
+          a1 = *reinterpret_cast<const float*>(lane_table + ob);
+          l1 = *reinterpret_cast<const float*>(lane_table + ob + 128);
         } else {
-          ia = ((cw.x >> (4 * i)) & 15u) | (phase_raw<PCB>(pw, i) << 4);
-          ib = ((cw.y >> (4 * i)) & 15u) | (phase_raw<PCB>(pw, i + 8) << 4);
+          const float2 al0 = lutAL[((cw.x >> (4 * i)) & 15u) | (phase_raw<PCB>(pw, i) << 4)];
+          const float2 al1 = lutAL[((cw.y >> (4 * i)) & 15u) | (phase_raw<PCB>(pw, i + 8) << 4)];
+          a0 = al0.x, a1 = al1.x, l0 = al0.y, l1 = al1.y;
         }
-        const float2 al0 = lutAL[ia], al1 = lutAL[ib];
-        const float a0 = al0.x, a1 = al1.x, l0 = al0.y, l1 = al1.y;
         f32x2 nl2;                                               // -(lr * d) of the pair
         if constexpr (DIR == 2) {
           const float g0 = gv[i], g1 = gv[i + 8];
@@ -662,7 +870,6 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
           nl2 = pk(g0 == 0.0f ? 0.0f : n0, g1 == 0.0f ? 0.0f : n1);
         } else {
           const float g0 = gv[i], g1 = gv[i + 8];
-          ok = ok && fabsf(g0) >= g_lo && fabsf(g0) <= g_hi && fabsf(g1) >= g_lo && fabsf(g1) <= g_hi;
           f32x2 u = pk(g0, g1);
           if constexpr (DIR == 3) u = div2p(u, nden2[i], rden2[i]);
           if (use_div) u = div2p(u, ndiv2, rdiv2);
@@ -704,46 +911,74 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
         }
       }
       ok = ok && s_new <= 4.0f * s_old && s_old <= 4.0f * s_new;
-      if (!ok) {                                                // rare: values outside the unchecked divisions' range
-        update_group_general<PCB, DIR, GT>(T, r, cg, denom, div, use_div, lutAL, plut, P);
-        continue;
-      }
-      T.scales_out[r * scale_stride + cg] = static_cast<uint8_t>(sb_new);
-
       // ---- projection back to (code, phase) (bitlattice/reference.py:250-274, 324-334)
       const uint32_t h0 = (T.offset + static_cast<uint32_t>(static_cast<uint64_t>(r) * cols + cg * 16)) * 0x27D4EB2Fu +
                           T.key;
       const f32x2 nsnew2 = pk(-s_new, -s_new), rsnew2 = pk(inv_new, inv_new);
       uint2 cout = make_uint2(0u, 0u);
       PW pout{};
+      if constexpr (kNarrow) {
+        uint32_t z = 0u, pe[2], po[2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float tv[2];
-        upk(div2p(mul2p(tau2[i], sold2), nsnew2, rsnew2), tv[0], tv[1]);
-        // nearest levels of the pair through the hardware conversion (ties to even: see the notes above). It
-        // saturates, and beyond the last level the table's factor is 0, so a target outside [-6, 6] needs no clamp
-        // (the range check has made it finite): its phase coordinate is 0 either way.
-        const uint32_t near2 = cvt_e2m1x2(tv[1], tv[0]);
+        for (int par = 0; par < 2; ++par) {                     // elements of even, then of odd index
+          uint32_t S[2][4], sg[2][4];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float t = tv[e];
-          const uint32_t nib = e == 0 ? (near2 & 15u) : (near2 >> 4);
-          const float4 L = plut24[nib];
-          // phase coordinate times half, in 2^-24 fixed point (exact scaling; |q| <= 64, so it fits 31 bits); the
-          // draw n = hash >> 8 rounds up iff n * 2^-24 < frac(q), i.e. iff n < ceil(frac(q) * 2^24): the carry of
-          // adding 2^24 - 1 - n to ceil(q * 2^24). k = floor(q) + carry, two's complement.
-          const int q24 = __float2int_ru((t - L.x) * (t < L.x ? L.z : L.y));
-          uint32_t h = h0 + static_cast<uint32_t>(i + 8 * e) * 0x27D4EB2Fu;
-          h = (h ^ (h >> 16)) * 0x7FEB352Du;
-          h = (h ^ (h >> 15)) * 0x846CA68Bu;
-          h = ~(h ^ (h >> 16));
-          const int k = (q24 + static_cast<int>(h >> 8)) >> 24;
-          const uint32_t code = k == half_i ? __float_as_uint(L.w) : nib;      // +half: the level above, phase -half
-          if (e == 0) cout.x += code << (4 * i);
-          else cout.y += code << (4 * i);
-          phase_put<PCB>(pout, i + 8 * e, static_cast<uint32_t>(k) & pmask);
+          for (int k = 0; k < 4; ++k) {
+            const int i = 2 * k + par;
+            float t0, t1;
+            upk(div2p(mul2p(tau2[i], sold2), nsnew2, rsnew2), t0, t1);
+            project_pair(t0, t1, h0 + static_cast<uint32_t>(i) * 0x27D4EB2Fu, h0 + static_cast<uint32_t>(i + 8) * 0x27D4EB2Fu,
+                         spread, byte256, S[0][k], S[1][k], z);
+            sg[0][k] = __float_as_uint(t0);
+            sg[1][k] = __float_as_uint(t1);
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t c, p;
+            split_levels(S[h], sg[h], P.pb, half4, pmask4, c, p);
+            uint32_t& out = h == 0 ? cout.x : cout.y;
+            out = par == 0 ? c : out + c * 16u;
+            (par == 0 ? pe[h] : po[h]) = p;
+          }
+        }
+        ok = ok && z < kUndecided;
+        if constexpr (PCB == 4) pout = make_uint2(join_phases<4>(pe[0], po[0]), join_phases<4>(pe[1], po[1]));
+        else pout = static_cast<PW>(join_phases<PCB>(pe[0], po[0]) | (join_phases<PCB>(pe[1], po[1]) << (8 * PCB)));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          float tv[2];
+          upk(div2p(mul2p(tau2[i], sold2), nsnew2, rsnew2), tv[0], tv[1]);
+          // nearest levels of the pair through the hardware conversion (ties to even: see the notes above). It
+          // saturates, and beyond the last level the table's factor is 0, so a target outside [-6, 6] needs no clamp
+          // (the range check has made it finite): its phase coordinate is 0 either way.
+          const uint32_t near2 = cvt_e2m1x2(tv[1], tv[0]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float t = tv[e];
+            const uint32_t nib = e == 0 ? (near2 & 15u) : (near2 >> 4);
+            const float4 L = plut24[nib];
+            // phase coordinate times half, in 2^-24 fixed point (exact scaling; |q| <= 64, so it fits 31 bits); the
+            // draw n = hash >> 8 rounds up iff n * 2^-24 < frac(q), i.e. iff n < ceil(frac(q) * 2^24): the carry of
+            // adding 2^24 - 1 - n to ceil(q * 2^24). k = floor(q) + carry, two's complement.
+            const int q24 = __float2int_ru((t - L.x) * (t < L.x ? L.z : L.y));
+            uint32_t h = h0 + static_cast<uint32_t>(i + 8 * e) * 0x27D4EB2Fu;
+            h = (h ^ (h >> 16)) * 0x7FEB352Du;
+            h = (h ^ (h >> 15)) * 0x846CA68Bu;
+            h = ~(h ^ (h >> 16));
+            const int k = (q24 + static_cast<int>(h >> 8)) >> 24;
+            const uint32_t code = k == half_i ? __float_as_uint(L.w) : nib;      // +half: the level above, phase -half
+            if (e == 0) cout.x += code << (4 * i);
+            else cout.y += code << (4 * i);
+            phase_put<PCB>(pout, i + 8 * e, static_cast<uint32_t>(k) & pmask);
+          }
         }
       }
+      if (!ok) {      // rare: values outside the unchecked divisions' range, or a draw next to its threshold
+        update_group_general<PCB, DIR, GT>(T, r, cg, denom, div, use_div, lutAL, plut, P);
+        continue;
+      }
+      T.scales_out[r * scale_stride + cg] = static_cast<uint8_t>(sb_new);
       cout.x = e2m1_drop_negative_zero(cout.x);
       cout.y = e2m1_drop_negative_zero(cout.y);
       *reinterpret_cast<uint2*>(T.codes + r * code_stride + cg * 8) = cout;
@@ -837,6 +1072,7 @@ static StepParams make_params(double lr, double decay, int pb, int rule, double 
   P.r_hi = static_cast<float>(exp(kappa));
   P.mode = rounding;
   P.strat_k = static_cast<float>(strat_k > 0 ? strat_k : 1);
+  P.rows_per_thread = 1;
   return P;
 }
 
@@ -863,6 +1099,16 @@ static TensorDesc make_desc(uint8_t* codes, uint8_t* phase, const uint8_t* scale
   return d;
 }
 
+template <int PCB, int DIR, typename GT>
+static void launch_update_fast(unsigned blocks, cudaStream_t st, const Batch& B, unsigned char* scratch, int has_stats,
+                               const StepParams& P) {
+  constexpr int kSmem = kLaneTableBytes<PCB> + RowSlots<PCB, GT>::kTotal;
+  auto kernel = update_kernel<PCB, DIR, GT, true>;
+  // (a failure is the launcher's cudaGetLastError)
+  if (kSmem > 40960 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return;
+  kernel<<<blocks, kThreads, kSmem, st>>>(B, scratch, has_stats, P);
+}
+
 template <int DIR, typename GT, bool FAST>
 static void launch_update_pcb(int pcb, unsigned blocks, cudaStream_t st, const Batch& B, unsigned char* scratch,
                               int has_stats, const StepParams& P) {
@@ -870,19 +1116,50 @@ static void launch_update_pcb(int pcb, unsigned blocks, cudaStream_t st, const B
     case 0:
       if constexpr (!FAST) update_kernel<0, DIR, GT, false><<<blocks, kThreads, 0, st>>>(B, scratch, has_stats, P);
       break;
-    case 1: update_kernel<1, DIR, GT, FAST><<<blocks, kThreads, 0, st>>>(B, scratch, has_stats, P); break;
-    case 2: update_kernel<2, DIR, GT, FAST><<<blocks, kThreads, 0, st>>>(B, scratch, has_stats, P); break;
-    case 4: update_kernel<4, DIR, GT, FAST><<<blocks, kThreads, 0, st>>>(B, scratch, has_stats, P); break;
+    case 1:
+      if constexpr (FAST) launch_update_fast<1, DIR, GT>(blocks, st, B, scratch, has_stats, P);
+      else update_kernel<1, DIR, GT, false><<<blocks, kThreads, 0, st>>>(B, scratch, has_stats, P);
+      break;
+    case 2:
+      if constexpr (FAST) launch_update_fast<2, DIR, GT>(blocks, st, B, scratch, has_stats, P);
+      else update_kernel<2, DIR, GT, false><<<blocks, kThreads, 0, st>>>(B, scratch, has_stats, P);
+      break;
+    case 4:
+      if constexpr (FAST) launch_update_fast<4, DIR, GT>(blocks, st, B, scratch, has_stats, P);
+      else update_kernel<4, DIR, GT, false><<<blocks, kThreads, 0, st>>>(B, scratch, has_stats, P);
+      break;
     default: update_kernel<8, DIR, GT, FAST><<<blocks, kThreads, 0, st>>>(B, scratch, has_stats, P); break;
   }
+}
+
+// Rows a thread walks, for the whole batch: few enough that every SM gets its two CTAs (a 1024 x 1024 weight has 256 CTAs
+// of one row per thread and 32 of eight), enough that what a CTA does first -- its tables, its columns' denominators, about
+// a row and a half -- is shared, and so that the last wave is not nearly empty: the number that minimises
+// waves * (rows + 3/2).
+static int choose_rows_per_thread(const Batch& B, int sms) {
+  static const int kRows[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 28, 32, 36, 40, 44, 48, 56, 64};
+  const int64_t slots = 2 * static_cast<int64_t>(sms);
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int r : kRows) {
+    int64_t blocks = 0;
+    for (int i = 0; i < B.count; ++i) blocks += update_blocks(B.t[i].rows, B.t[i].cols, r);
+    const int64_t cost = (blocks + slots - 1) / slots * (2 * r + 3);
+    if (cost < best_cost) best = r, best_cost = cost;
+    if (blocks <= slots) break;
+  }
+  return best;
 }
 
 // dir: 0 = D given (fp32), else BL_DIR_* + 1
 template <typename GT>
 static int launch_update(int dir, int pcb, cudaStream_t st, const Batch& B, unsigned char* scratch, int has_stats,
-                         const StepParams& P) {
+                         StepParams P) {
   int64_t blocks = 0;
-  for (int i = 0; i < B.count; ++i) blocks += update_blocks(B.t[i].rows, B.t[i].cols);
+  int device = 0;
+  BL_CUDA(cudaGetDevice(&device));
+  P.rows_per_thread = choose_rows_per_thread(B, sm_count(device));
+  for (int i = 0; i < B.count; ++i) blocks += update_blocks(B.t[i].rows, B.t[i].cols, P.rows_per_thread);
   BL_REQUIRE(blocks > 0 && blocks <= 0x7FFFFFFF, "lattice update: too many blocks (%lld)", (long long)blocks);
   const unsigned nb = static_cast<unsigned>(blocks);
   const bool fast = P.mode == BL_ROUND_SR && P.pb >= 1 && P.pb <= 7 && g_update_route.load(std::memory_order_relaxed) == 0;

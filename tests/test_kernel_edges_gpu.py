@@ -138,3 +138,36 @@ def test_tile_gemm_few_rows(M, N, K):
         _ops.gemm_select("auto")
     assert torch.equal(outs[0], outs[1]) and outs[0].isfinite().all()
     assert _ops.gemm_status(0) == 0
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4])
+@pytest.mark.parametrize("direction,dtype,lr", [("colnorm", torch.bfloat16, 3e-3), ("sign", torch.float32, 0.5),
+                                                ("raw", torch.float16, 40.0)])
+@pytest.mark.parametrize("rows,cols", [(1, 16), (37, 48), (300, 4112)])
+def test_update_projection_edges(rows, cols, direction, dtype, lr, bits):
+    """The fast update with 1 to 4 phase bits against the general route (the reference's arithmetic step by step), bit for
+    bit: every code and phase, single groups, rows that end inside a block, targets beyond the last level (large lr),
+    zero gradients (a group of them leaves the fast route), several steps so that rows are walked and carried over."""
+    gen = torch.Generator(device="cuda").manual_seed(bits * rows + cols)
+    cb = _ops.phase_container(bits)
+    codes = torch.randint(0, 256, (rows, cols // 2), dtype=torch.uint8, device="cuda", generator=gen)
+    scales = torch.randint(0x20, 0x48, (rows, cols // 16), dtype=torch.uint8, device="cuda", generator=gen)
+    mask = sum(((1 << bits) - 1) << s for s in range(0, 8, cb))
+    phase = torch.randint(0, 256, (rows, cols * cb // 8), dtype=torch.uint8, device="cuda", generator=gen) & mask
+    grad = (torch.randn(rows, cols, device="cuda", generator=gen) * 1e-2).to(dtype)
+    grad[:, 5] = 0 if rows == 37 else grad[:, 5]
+    gs = torch.tensor([0.02], device="cuda")
+    ends = []
+    try:
+        for route in ("auto", "general"):
+            _ops.update_select(route)
+            c, p, s = codes.clone(), phase.clone(), scales.clone()
+            for step in (1, 2, 3):
+                _ops.lattice_update(c, p, s, gs, None, grad, "nvfp4", rows, cols, lr=lr, weight_decay=0.0, phase_bits=bits,
+                                    phase_cb=cb, rounding="sr", seed=77, step=step, strata=16, scale_rule="fit", trust=0.1,
+                                    trust_lr=0.0, direction=direction)
+            ends.append((c, p, s))
+    finally:
+        _ops.update_select("auto")
+    for a, b in zip(*ends):
+        assert torch.equal(a, b)
