@@ -502,15 +502,17 @@ def fp4_fold_scales(scales: torch.Tensor, row_tiles: int, piece: torch.Tensor, g
 
 
 def quantize_nvfp4_t(x: torch.Tensor, hadamard: torch.Tensor | None, seed: int = -1, step: int = 0,
-                     global_scale: torch.Tensor | None = None, blocked: bool = False):
+                     global_scale: torch.Tensor | None = None, blocked: bool = False, pad_rows: int = 1):
     """x [M, K] -> NVFP4 of x^T (rotated by ``hadamard`` along M): (packed [K, M/2], scales, global [1])
-    (reference: torch.ops.bitlattice.quantize_nvfp4_t)."""
+    (reference: torch.ops.bitlattice.quantize_nvfp4_t). ``pad_rows``: x counts as followed by rows of zeros up to the next
+    multiple (M in the result's shapes is then that multiple), without a padded copy."""
     _require(x, "x")
     if x.dim() != 2:
         raise RuntimeError("x must be a contiguous 2-D CUDA tensor")
     if x.dtype not in _C.DTYPE:
         raise RuntimeError("x must be bf16, fp16 or fp32")
-    M, K = x.shape
+    rows, K = x.shape
+    M = -(-rows // pad_rows) * pad_rows
     if hadamard is not None:
         _require(hadamard, "hadamard", torch.float32)
         if hadamard.numel() != 256:
@@ -526,7 +528,7 @@ def quantize_nvfp4_t(x: torch.Tensor, hadamard: torch.Tensor | None, seed: int =
         _require(bound, "global_scale")
     else:
         amax = torch.empty(4, dtype=torch.float32, device=x.device)
-    _C.call("bl_nvfp4_quantize_t", _C.ptr(x), _C.DTYPE[x.dtype], M, K, _C.ptr(hadamard), int(seed),
+    _C.call("bl_nvfp4_quantize_t_rows", _C.ptr(x), _C.DTYPE[x.dtype], rows, M, K, _C.ptr(hadamard), int(seed),
             int(step) & 0xFFFFFFFF, _C.ptr(bound), _C.ptr(amax), _C.ptr(packed), _C.ptr(scales), _C.ptr(gout),
             int(blocked), _C.device_of(x), _C.stream_of(x), extra_kernels=0 if bound is not None else 1)
     return packed, scales if blocked else scales.view(torch.float8_e4m3fn), gout

@@ -298,7 +298,7 @@ __device__ __forceinline__ void rotate_half(const float raw[16], const float* __
 
 // amax of the (rotated) transposed tensor; out as for amax_kernel but without the scale
 template <typename T>
-__global__ void __launch_bounds__(kQThreads) amax_t_kernel(const T* __restrict__ x, int64_t M, int64_t K,
+__global__ void __launch_bounds__(kQThreads) amax_t_kernel(const T* __restrict__ x, int64_t rows, int64_t M, int64_t K,
                                                            const float* __restrict__ H, float* __restrict__ out) {
   __shared__ float sH[256];
   if (H != nullptr) sH[threadIdx.x] = H[threadIdx.x];
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kQThreads) amax_t_kernel(const T* __restrict__
     const int64_t k = t % K, mb = t / K;
     float raw[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) raw[i] = to_f<T>(x[(mb * 16 + i) * K + k]);
+    for (int i = 0; i < 16; ++i) raw[i] = mb * 16 + i < rows ? to_f<T>(x[(mb * 16 + i) * K + k]) : 0.0f;
     if (H == nullptr) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) m = fmaxf(m, fabsf(raw[i]));
@@ -343,10 +343,10 @@ __global__ void global_t_kernel(const float* __restrict__ in, int given, float* 
   global_out[0] = global_t(in, given);
 }
 
-// x [M, K] -> NVFP4 of x^T. A CTA stages a [128, 64] tile of x in shared memory with coalesced row reads; the work
+// x [rows, K], read as [M, K] with zeros below -> NVFP4 of x^T. A CTA stages a [128, 64] tile of x in shared memory with coalesced row reads; the work
 // item (k, mb, half) quantizes 8 of the 16 rotated values of block mb of column k; lane pairs (half 0/1) share a block.
 template <typename T, bool SR>
-__global__ void __launch_bounds__(kQThreads) quantize_t_kernel(const T* __restrict__ x, int64_t M, int64_t K,
+__global__ void __launch_bounds__(kQThreads) quantize_t_kernel(const T* __restrict__ x, int64_t rows, int64_t M, int64_t K,
                                                                const float* __restrict__ H,
                                                                const float* __restrict__ global, int given,
                                                                float* __restrict__ global_out, uint32_t key,
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(kQThreads) quantize_t_kernel(const T* __restri
   for (int i = threadIdx.x; i < kTM * kTK; i += kQThreads) {
     const int rr = i / kTK, cc = i % kTK;
     const int64_t m = m0 + rr, k = k0 + cc;
-    tile[rr][cc] = (m < M && k < K) ? to_f<T>(x[m * K + k]) : 0.0f;
+    tile[rr][cc] = (m < rows && k < K) ? to_f<T>(x[m * K + k]) : 0.0f;
   }
   __syncthreads();
   const float g = global_t(global, given);
@@ -438,9 +438,11 @@ __device__ __forceinline__ void rotate16_tree2(const f32x2 p[16], f32x2 v[16]) {
 
 // Transposed quantizer, one thread per (block of 16 rows, pair of adjacent columns); adjacent lanes read adjacent column
 // pairs, so every row of the tile is read as full 128-byte lines; codes and scales of the 64 x 128 tile are staged in
-// shared memory and written out as rows of the transposed result.
+// shared memory and written out as rows of the transposed result. Rows from `rows` on (where the caller's row count is no
+// multiple of the GEMM's granularity) count as zeros and are not read: a padded copy of x cost two more passes
+// (95 us for 4999 x 25600 fp16, beside 27 to 161 us for the quantizer itself).
 template <typename T, bool SR>
-__global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __restrict__ x, int64_t M, int64_t K,
+__global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __restrict__ x, int64_t rows, int64_t M, int64_t K,
                                                                 const float* __restrict__ H,
                                                                 const float* __restrict__ global, int given,
                                                                 float* __restrict__ global_out, uint32_t key,
@@ -465,8 +467,16 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
   if (active) {
     float ra[16], rb[16];
     const T* p = x + m * K + k;
+    if (m + 16 <= rows) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) load2(p + i * K, ra[i], rb[i]);
+      for (int i = 0; i < 16; ++i) load2(p + i * K, ra[i], rb[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        ra[i] = rb[i] = 0.0f;
+        if (m + i < rows) load2(p + i * K, ra[i], rb[i]);
+      }
+    }
     const float g = global_t(global, given);
     if (global_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) global_out[0] = g;
     const float rg = __frcp_rn(g);
@@ -484,8 +494,8 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
       // route takes no registers from the usual one
       float wait[32];
       for (int i = 0; i < 16; ++i) {
-        wait[2 * i] = to_f<T>(p[i * K]);
-        wait[2 * i + 1] = to_f<T>(p[i * K + 1]);
+        wait[2 * i] = m + i < rows ? to_f<T>(p[i * K]) : 0.0f;
+        wait[2 * i + 1] = m + i < rows ? to_f<T>(p[i * K + 1]) : 0.0f;
       }
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
@@ -926,12 +936,12 @@ extern "C" int bl_nvfp4_quantize_4over6(const void* x, int dtype, int64_t rows, 
 }
 
 template <typename T>
-static int quantize_t_typed(const T* x, int64_t M, int64_t K, const float* H, int64_t seed, uint32_t step,
+static int quantize_t_typed(const T* x, int64_t rows, int64_t M, int64_t K, const float* H, int64_t seed, uint32_t step,
                             const float* bound, float* amax_scratch, uint8_t* codes, uint8_t* scales, float* gout,
                             int layout, int device, cudaStream_t st) {
   if (bound == nullptr) {
     BL_CUDA(cudaMemsetAsync(amax_scratch, 0, 16, st));
-    amax_t_kernel<<<grid_for((M / 16) * K, kQThreads, device), kQThreads, 0, st>>>(x, M, K, H, amax_scratch);
+    amax_t_kernel<<<grid_for((M / 16) * K, kQThreads, device), kQThreads, 0, st>>>(x, rows, M, K, H, amax_scratch);
     BL_CUDA(cudaGetLastError());
   }
   const float* src = bound == nullptr ? amax_scratch : bound;
@@ -947,20 +957,21 @@ static int quantize_t_typed(const T* x, int64_t M, int64_t K, const float* H, in
   const dim3 grid(static_cast<unsigned>((K + kTK - 1) / kTK), static_cast<unsigned>((M + kTM - 1) / kTM));
   const uint32_t key = seed < 0 ? 0u : hash_key(static_cast<uint32_t>(seed), step);
   const bool pairs = K % 2 == 0 && (reinterpret_cast<uintptr_t>(x) % (2 * sizeof(T))) == 0;
-  if (pairs && seed < 0) quantize_t3_kernel<T, false><<<grid, kQThreads, 0, st>>>(x, M, K, H, src, given, publish, key, codes, scales, layout);
-  else if (pairs) quantize_t3_kernel<T, true><<<grid, kQThreads, 0, st>>>(x, M, K, H, src, given, publish, key, codes, scales, layout);
-  else if (seed < 0) quantize_t_kernel<T, false><<<grid, kQThreads, 0, st>>>(x, M, K, H, src, given, publish, key, codes, scales, layout);
-  else quantize_t_kernel<T, true><<<grid, kQThreads, 0, st>>>(x, M, K, H, src, given, publish, key, codes, scales, layout);
+  if (pairs && seed < 0) quantize_t3_kernel<T, false><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, publish, key, codes, scales, layout);
+  else if (pairs) quantize_t3_kernel<T, true><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, publish, key, codes, scales, layout);
+  else if (seed < 0) quantize_t_kernel<T, false><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, publish, key, codes, scales, layout);
+  else quantize_t_kernel<T, true><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, publish, key, codes, scales, layout);
   BL_CUDA(cudaGetLastError());
   return 0;
 }
 
-extern "C" int bl_nvfp4_quantize_t(const void* x, int dtype, int64_t M, int64_t K, const float* H, int64_t seed,
-                                   uint32_t step, const float* global_bound, float* amax_scratch, uint8_t* codes,
-                                   uint8_t* scales, float* global_out, int sf_layout, int device, bl_stream_t stream) {
+extern "C" int bl_nvfp4_quantize_t_rows(const void* x, int dtype, int64_t rows, int64_t M, int64_t K, const float* H, int64_t seed,
+                                        uint32_t step, const float* global_bound, float* amax_scratch, uint8_t* codes,
+                                        uint8_t* scales, float* global_out, int sf_layout, int device, bl_stream_t stream) {
   BL_REQUIRE(x && codes && scales && global_out, "quantize_nvfp4_t: null buffer");
   BL_REQUIRE(M > 0 && K > 0 && M % 16 == 0, "quantize_nvfp4_t: rows must be a multiple of 16, got %lld x %lld",
              (long long)M, (long long)K);
+  BL_REQUIRE(rows > 0 && rows <= M, "quantize_nvfp4_t: %lld rows present of %lld", (long long)rows, (long long)M);
   BL_REQUIRE((M / 16) <= 65535 * 8, "quantize_nvfp4_t: too many rows (%lld)", (long long)M);
   BL_REQUIRE(global_bound != nullptr || amax_scratch != nullptr,
              "quantize_nvfp4_t: without a scale bound the amax pass needs a 4-float scratch buffer");
@@ -972,10 +983,17 @@ extern "C" int bl_nvfp4_quantize_t(const void* x, int dtype, int64_t M, int64_t 
   if (sf_layout == BL_SF_BLOCKED && blocked_needs_padding(K, M / 16))
     BL_CUDA(cudaMemsetAsync(scales, 0, bl_blocked_scale_bytes(K, M / 16), st));
   if (dtype == BL_BF16)
-    return quantize_t_typed(static_cast<const __nv_bfloat16*>(x), M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
+    return quantize_t_typed(static_cast<const __nv_bfloat16*>(x), rows, M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
   if (dtype == BL_F16)
-    return quantize_t_typed(static_cast<const __half*>(x), M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
-  return quantize_t_typed(static_cast<const float*>(x), M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
+    return quantize_t_typed(static_cast<const __half*>(x), rows, M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
+  return quantize_t_typed(static_cast<const float*>(x), rows, M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
+}
+
+extern "C" int bl_nvfp4_quantize_t(const void* x, int dtype, int64_t M, int64_t K, const float* H, int64_t seed,
+                                   uint32_t step, const float* global_bound, float* amax_scratch, uint8_t* codes,
+                                   uint8_t* scales, float* global_out, int sf_layout, int device, bl_stream_t stream) {
+  return bl_nvfp4_quantize_t_rows(x, dtype, M, M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out,
+                                  sf_layout, device, stream);
 }
 
 extern "C" int bl_nvfp4_requantize_t(const uint8_t* codes, const uint8_t* scales, const float* global_scale, int64_t N,

@@ -349,7 +349,7 @@ class SharedInputFp4Linears(torch.autograd.Function):
                                      lambda: backend._input_operands(x, recipe, site=backend._site(weights[0], "x")))
         else:
             xq, xt = backend._shared(x, recipe, "fwd", lambda: backend._act_operand(
-                backend._pad_rows(x.reshape(-1, K), 16).contiguous(), recipe)), None
+                backend._flat_rows(x, 16), recipe)), None
         ctx.weights, ctx.recipe, ctx.xt = weights, recipe, xt
         ctx.x_meta = (x.shape, x.dtype)
         return tuple(backend.fp4_mm(xq, backend.weight_operand(w), x.dtype)[:M].reshape(*x.shape[:-1], w.shape[0])
@@ -374,7 +374,7 @@ class SharedInputFp4Linears(torch.autograd.Function):
                     gx, g2p, gq = backend.fp4_dgrad(gy, w, ctx.recipe)
                     gx_sum = gx if gx_sum is None else gx_sum.add_(gx)
             else:
-                g2p, gq = backend._pad_rows(gy.reshape(-1, gy.shape[-1]), 32).contiguous(), None
+                g2p, gq = backend._flat_rows(gy, 32), None
             staged.append((g2p, gq))
         gws = []
         for i, (w, st) in enumerate(zip(ctx.weights, staged)):

@@ -4,7 +4,8 @@ import pytest
 import torch
 
 import oracle
-from bitlattice_b200 import _C, _ops
+import bitlattice_b200 as bl
+from bitlattice_b200 import _C, _ops, backend
 
 pytestmark = pytest.mark.gpu
 
@@ -170,4 +171,45 @@ def test_update_projection_edges(rows, cols, direction, dtype, lr, bits):
     finally:
         _ops.update_select("auto")
     for a, b in zip(*ends):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("seed", [-1, 7])
+@pytest.mark.parametrize("rows,K,rotate,bound", [(1, 16, True, True), (17, 130, True, True), (33, 64, False, True),
+                                                 (127, 192, True, False), (129, 95, True, True), (300, 1000, "other", True)])
+def test_quantize_t_ragged_rows(rows, K, rotate, bound, seed):
+    """Rows missing from the last block count as zeros: the bytes of the padded tensor, on the paired and the odd-width
+    kernel, with the structured rotation, another matrix and none, with a bound and with the amax pass."""
+    gen = torch.Generator(device="cuda").manual_seed(rows * K)
+    x = torch.randn(rows, K, device="cuda", generator=gen).to(torch.bfloat16)
+    padded = torch.nn.functional.pad(x, (0, 0, 0, -rows % 32))
+    H = (torch.randn(16, 16, device="cuda", generator=gen) if rotate == "other"
+         else backend._hadamard16(x.device, torch.float32) if rotate else None)
+    g = torch.tensor([2e-3], device="cuda") if bound else None
+    want = _ops.quantize_nvfp4_t(padded, H, seed, 0, g, blocked=True)
+    got = _ops.quantize_nvfp4_t(x, H, seed, 0, g, blocked=True, pad_rows=32)
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+
+
+@pytest.mark.parametrize("recipe", ["nvidia", "4over6"])
+@pytest.mark.parametrize("rows", [1, 13, 100])
+def test_ragged_rows_of_a_layer(rows, recipe):
+    """A layer on a row count that is no multiple of 32, starting at an address that is no multiple of 16: outputs and both
+    gradients are those of the rows padded with zeros."""
+    recipe = backend.FP4_RECIPES[recipe]
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    w = bl.LatticeTensor.from_float(torch.randn(96, 64, device="cuda", generator=gen) * 0.02, "nvfp4", dtype=torch.bfloat16)
+
+    def shifted(cols):
+        return torch.randn(rows * cols + 1, device="cuda", generator=gen).to(torch.bfloat16)[1:].view(rows, cols)
+    x, gy = shifted(64), shifted(96)
+    outs = []
+    for pad in (0, -rows % 32):
+        backend.set_sr_seed(5)
+        xi, gi = (torch.nn.functional.pad(t, (0, 0, 0, pad)) if pad else t for t in (x, gy))
+        y, xt = backend.fp4_forward_saving(xi, w, None, recipe)
+        gx, gw = backend.fp4_backward(gi, w, xt, True, True, recipe)
+        outs.append((y[:rows], gx[:rows], gw, backend.nvfp4_linear(xi, w, None, recipe)[:rows]))
+    for a, b in zip(*outs):
         assert torch.equal(a, b)
