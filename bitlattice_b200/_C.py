@@ -66,7 +66,7 @@ _SIGNATURES = {
     "bl_nvfp4_quantize_t": (_c.c_int, [_P, _c.c_int, _c.c_int64, _c.c_int64, _P, _c.c_int64, _c.c_uint32, _P, _P, _P,
                                        _P, _P, _c.c_int, _c.c_int, _P]),
     "bl_nvfp4_quantize_t_rows": (_c.c_int, [_P, _c.c_int, _c.c_int64, _c.c_int64, _c.c_int64, _P, _c.c_int64, _c.c_uint32, _P,
-                                            _P, _P, _P, _P, _c.c_int, _c.c_int, _P]),
+                                            _c.c_float, _P, _P, _P, _P, _c.c_int, _c.c_int, _P]),
     "bl_nvfp4_requantize_t": (_c.c_int, [_P, _P, _P, _c.c_int64, _c.c_int64, _P, _P, _P, _c.c_int, _c.c_int, _P]),
     "bl_blocked_scale_bytes": (_c.c_size_t, [_c.c_int64, _c.c_int64]),
     "bl_nvfp4_scales_to_blocked": (_c.c_int, [_P, _c.c_int64, _c.c_int64, _P, _c.c_int, _P]),
@@ -168,6 +168,20 @@ class Counters:
         """(total milliseconds, calls) of a timed entry point; synchronize the device first."""
         ev = cls.events.get(name, [])
         return sum(a.elapsed_time(b) for a, b in ev), len(ev)
+
+
+def native(name: str, fn, *args, extra_kernels: int = 0):
+    """``fn(*args)``, a function of the extension module that calls the entry point ``name``, counted as ``call`` counts."""
+    if Counters.timed is not None and name in Counters.timed:
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        out = fn(*args)
+        b.record()
+        Counters.events.setdefault(name, []).append((a, b))
+    else:
+        out = fn(*args)
+    Counters.launches += KERNELS_PER_CALL.get(name, 0) + extra_kernels
+    return out
 
 
 def call(name: str, *args, extra_kernels: int = 0) -> None:

@@ -14,6 +14,7 @@ importing the package loads it and fails if it has not been built (``python bitl
 from . import _C
 
 _C.lib()          # fail loudly here, not at the first kernel call, when the CUDA library is missing
+from . import _host  # noqa: E402, F401  (the same for the extension module, built by the same script)
 
 from . import backend, formats, io, optim, packing, parallel  # noqa: E402
 from ._ops import HAVE_EXT  # noqa: E402

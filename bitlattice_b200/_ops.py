@@ -12,7 +12,7 @@ import math
 
 import torch
 
-from . import _C
+from . import _C, _host
 from . import formats as F
 
 HAVE_EXT = True            # the library is mandatory; importing this package fails without it (see _C.lib)
@@ -81,15 +81,9 @@ def dequantize(packed, scales, global_scale, zeros, fmt, rows: int, cols: int, d
     """Dense [rows, cols] tensor of the represented values (reference: bitlattice/_ops.py:55-61)."""
     if zeros is not None or not _is_nvfp4(fmt):
         raise RuntimeError("only NVFP4 tensors (no zero points) are built")
-    _require(packed, "packed", torch.uint8)
-    _require(scales, "scales")
-    _require(global_scale, "global_scale", torch.float32)
     if dtype not in _C.DTYPE:
         raise RuntimeError(f"dequantize to {dtype} is not built (float32, bfloat16, float16 are)")
-    out = torch.empty(rows, cols, dtype=dtype, device=packed.device)
-    _C.call("bl_nvfp4_dequantize", _C.ptr(packed), _C.ptr(scales), _C.ptr(global_scale), rows, cols, _C.ptr(out),
-            _C.DTYPE[dtype], _C.device_of(packed), _C.stream_of(packed))
-    return out
+    return _C.native("bl_nvfp4_dequantize", _host.dequantize, packed, scales, global_scale, rows, cols, _C.DTYPE[dtype])
 
 
 # ------------------------------------------------------------------------------------------------ lattice update
@@ -373,10 +367,7 @@ def amax_global(x: torch.Tensor) -> torch.Tensor:
     """fp32 [4]: [0] = max|x|, [1] = the per-tensor NVFP4 scale max(amax/(6*448), 1e-12)
     (reference: bitlattice/backend.py:240-241), [3] = max(amax/(6*256), 1e-12), the per-tensor scale of the
     four-over-six recipe."""
-    _require(x, "x")
-    out = torch.empty(4, dtype=torch.float32, device=x.device)
-    _C.call("bl_nvfp4_amax", _C.ptr(x), _C.DTYPE[x.dtype], x.numel(), _C.ptr(out), _C.device_of(x), _C.stream_of(x))
-    return out
+    return _C.native("bl_nvfp4_amax", _host.amax_global, x)
 
 
 def _scale_buffer(rows: int, cols16: int, blocked: bool, device) -> torch.Tensor:
@@ -404,16 +395,7 @@ def quantize_nvfp4(x: torch.Tensor, global_scale: torch.Tensor, seed: int = -1, 
 def amax_quantize_nvfp4(x: torch.Tensor, seed: int = -1, step: int = 0, blocked: bool = False):
     """``amax_global`` and ``quantize_nvfp4`` against the scale it finds, enqueued by one library call: returns
     (packed, scales, amax [4]); the per-tensor scale is ``amax[1:2]``."""
-    _require(x, "x")
-    if x.dtype not in _C.DTYPE:
-        raise RuntimeError("x must be bf16, fp16 or fp32")
-    cols = x.shape[-1]
-    rows = x.numel() // cols
-    am = torch.empty(4, dtype=torch.float32, device=x.device)
-    packed = torch.empty(rows, cols // 2, dtype=torch.uint8, device=x.device)
-    scales = _scale_buffer(rows, cols // 16, blocked, x.device)
-    _C.call("bl_nvfp4_amax_quantize", _C.ptr(x), _C.DTYPE[x.dtype], rows, cols, _C.ptr(am), int(seed),
-            int(step) & 0xFFFFFFFF, _C.ptr(packed), _C.ptr(scales), int(blocked), _C.device_of(x), _C.stream_of(x))
+    packed, scales, am = _C.native("bl_nvfp4_amax_quantize", _host.amax_quantize, x, seed, step, blocked)
     return packed, scales if blocked else scales.view(torch.float8_e4m3fn), am
 
 
@@ -422,18 +404,9 @@ def quantize_nvfp4_4over6(x: torch.Tensor, global_scale: torch.Tensor, select: s
     mapped to 6" and "maximum mapped to 4" (``select``: 'mse' or 'mae'). ``global_scale``: amax / (6 * 256), i.e.
     ``amax_global(x)[3:4]`` (reference: torch.ops.bitlattice.nvfp4_quantize with four_over_six; Python twin
     bitlattice/fp4ref.py:103-135)."""
-    _require(x, "x")
-    _require(global_scale, "global_scale", torch.float32)
-    if x.dtype not in _C.DTYPE:
-        raise RuntimeError("x must be bf16, fp16 or fp32")
     if select not in ("mse", "mae"):
         raise ValueError("select must be 'mse' or 'mae'")
-    cols = x.shape[-1]
-    rows = x.numel() // cols
-    packed = torch.empty(rows, cols // 2, dtype=torch.uint8, device=x.device)
-    scales = _scale_buffer(rows, cols // 16, blocked, x.device)
-    _C.call("bl_nvfp4_quantize_4over6", _C.ptr(x), _C.DTYPE[x.dtype], rows, cols, _C.ptr(global_scale),
-            1 if select == "mae" else 0, _C.ptr(packed), _C.ptr(scales), int(blocked), _C.device_of(x), _C.stream_of(x))
+    packed, scales = _C.native("bl_nvfp4_quantize_4over6", _host.quantize_4over6, x, global_scale, select == "mae", blocked)
     return packed, scales if blocked else scales.view(torch.float8_e4m3fn)
 
 
@@ -502,64 +475,27 @@ def fp4_fold_scales(scales: torch.Tensor, row_tiles: int, piece: torch.Tensor, g
 
 
 def quantize_nvfp4_t(x: torch.Tensor, hadamard: torch.Tensor | None, seed: int = -1, step: int = 0,
-                     global_scale: torch.Tensor | None = None, blocked: bool = False, pad_rows: int = 1):
+                     global_scale: torch.Tensor | None = None, blocked: bool = False, pad_rows: int = 1,
+                     bound_factor: float = 1.0):
     """x [M, K] -> NVFP4 of x^T (rotated by ``hadamard`` along M): (packed [K, M/2], scales, global [1])
     (reference: torch.ops.bitlattice.quantize_nvfp4_t). ``pad_rows``: x counts as followed by rows of zeros up to the next
-    multiple (M in the result's shapes is then that multiple), without a padded copy."""
-    _require(x, "x")
-    if x.dim() != 2:
-        raise RuntimeError("x must be a contiguous 2-D CUDA tensor")
-    if x.dtype not in _C.DTYPE:
-        raise RuntimeError("x must be bf16, fp16 or fp32")
-    rows, K = x.shape
-    M = -(-rows // pad_rows) * pad_rows
-    if hadamard is not None:
-        _require(hadamard, "hadamard", torch.float32)
-        if hadamard.numel() != 256:
-            raise RuntimeError("hadamard must be a contiguous fp32 [16, 16] tensor")
-    packed = torch.empty(K, M // 2, dtype=torch.uint8, device=x.device)
-    scales = _scale_buffer(K, M // 16, blocked, x.device)
-    gout = torch.empty(1, dtype=torch.float32, device=x.device)
-    bound = amax = None
-    if global_scale is not None:
-        bound = global_scale
-        if bound.dtype != torch.float32 or bound.numel() != 1 or not bound.is_contiguous():
-            bound = bound.to(torch.float32).reshape(1).contiguous()
-        _require(bound, "global_scale")
-    else:
-        amax = torch.empty(4, dtype=torch.float32, device=x.device)
-    _C.call("bl_nvfp4_quantize_t_rows", _C.ptr(x), _C.DTYPE[x.dtype], rows, M, K, _C.ptr(hadamard), int(seed),
-            int(step) & 0xFFFFFFFF, _C.ptr(bound), _C.ptr(amax), _C.ptr(packed), _C.ptr(scales), _C.ptr(gout),
-            int(blocked), _C.device_of(x), _C.stream_of(x), extra_kernels=0 if bound is not None else 1)
+    multiple (M in the result's shapes is then that multiple), without a padded copy. ``bound_factor``: the bound is
+    ``global_scale * bound_factor``, multiplied in the kernel."""
+    packed, scales, gout = _C.native("bl_nvfp4_quantize_t", _host.quantize_t, x, hadamard, seed, step, global_scale,
+                                     bound_factor, blocked, pad_rows, extra_kernels=0 if global_scale is not None else 1)
     return packed, scales if blocked else scales.view(torch.float8_e4m3fn), gout
 
 
 def requantize_nvfp4_t(packed: torch.Tensor, scales: torch.Tensor, global_scale: torch.Tensor, blocked: bool = False):
     """NVFP4 W [N, K] -> NVFP4 of W^T: (packed [K, N/2], scales, global [1])
     (reference: torch.ops.bitlattice.requantize_nvfp4_t)."""
-    _require(packed, "packed", torch.uint8)
-    _require(scales, "scales")
-    g = global_scale
-    if g.dtype != torch.float32 or g.numel() != 1 or not g.is_contiguous():
-        g = g.to(torch.float32).reshape(1).contiguous()
-    _require(g, "global_scale")
-    N, K = packed.shape[0], packed.shape[1] * 2
-    out = torch.empty(K, N // 2, dtype=torch.uint8, device=packed.device)
-    osc = _scale_buffer(K, N // 16, blocked, packed.device)
-    gout = torch.empty(1, dtype=torch.float32, device=packed.device)
-    _C.call("bl_nvfp4_requantize_t", _C.ptr(packed), _C.ptr(scales), _C.ptr(g), N, K, _C.ptr(out), _C.ptr(osc),
-            _C.ptr(gout), int(blocked), _C.device_of(packed), _C.stream_of(packed))
+    out, osc, gout = _C.native("bl_nvfp4_requantize_t", _host.requantize_t, packed, scales, global_scale, blocked)
     return out, osc if blocked else osc.view(torch.float8_e4m3fn), gout
 
 
 def to_blocked(scales: torch.Tensor) -> torch.Tensor:
     """[rows, cols16] scale bytes -> flat 128x4-tiled layout (reference: bitlattice/backend.py:179-188)."""
-    _require(scales, "scales")
-    rows, cols16 = scales.shape
-    out = torch.empty(blocked_scale_bytes(rows, cols16), dtype=torch.uint8, device=scales.device)
-    _C.call("bl_nvfp4_scales_to_blocked", _C.ptr(scales), rows, cols16, _C.ptr(out), _C.device_of(scales),
-            _C.stream_of(scales))
-    return out
+    return _C.native("bl_nvfp4_scales_to_blocked", _host.to_blocked, scales)
 
 
 def assemble_gathered(recv: torch.Tensor, n: int, K: int, offsets):
@@ -585,27 +521,10 @@ def nvfp4_gemm(a_packed, a_sf, a_global, b_packed, b_sf, b_global, out_dtype=tor
     """(A B^T) * ga * gb for NVFP4 A [M, K], B [N, K] with blocked scales; fp32 accumulation on FP4 tensor cores
     (reference: bitlattice/backend.py:280-290). ``accumulate``: add the product to ``out`` (the bits of
     ``out + product`` as an add of two tensors of out's type)."""
-    _require(a_packed, "a_packed", torch.uint8)
-    _require(b_packed, "b_packed", torch.uint8)
-    _require(a_sf, "a_sf")
-    _require(b_sf, "b_sf")
-    M, K = a_packed.shape[0], a_packed.shape[1] * 2
-    N = b_packed.shape[0]
-    if b_packed.shape[1] * 2 != K:
-        raise RuntimeError(f"operand K mismatch: {K} vs {b_packed.shape[1] * 2}")
-    if a_sf.numel() < blocked_scale_bytes(M, K // 16) or b_sf.numel() < blocked_scale_bytes(N, K // 16):
-        raise RuntimeError("scale buffers are smaller than the blocked layout of their operands")
-    ga = _require(a_global, "a_global", torch.float32)
-    gb = _require(b_global, "b_global", torch.float32)
-    if out is None:
-        if accumulate:
-            raise RuntimeError("accumulate needs the tensor to add to (out=)")
-        out = torch.empty(M, N, dtype=out_dtype, device=a_packed.device)
-    elif out.shape != (M, N) or not out.is_cuda or out.stride(1) != 1:
-        raise RuntimeError(f"out must be a CUDA tensor [{M}, {N}] with unit column stride")
-    _C.call("bl_nvfp4_gemm_accumulate" if accumulate else "bl_nvfp4_gemm", _C.ptr(a_packed), _C.ptr(a_sf), _C.ptr(ga), _C.ptr(b_packed), _C.ptr(b_sf), _C.ptr(gb),
-            M, N, K, _C.ptr(out), _C.DTYPE[out.dtype], out.stride(0), _C.device_of(a_packed), _C.stream_of(a_packed))
-    return out
+    if out is None and out_dtype not in _C.DTYPE:
+        raise RuntimeError(f"gemm: output type {out_dtype} is not built (float32, bfloat16, float16 are)")
+    return _C.native("bl_nvfp4_gemm_accumulate" if accumulate else "bl_nvfp4_gemm", _host.gemm, a_packed, a_sf, a_global, b_packed,
+                     b_sf, b_global, _C.DTYPE.get(out_dtype, 0), out, accumulate)
 
 
 def swiglu_fwd(g: torch.Tensor, u: torch.Tensor) -> torch.Tensor:

@@ -14,6 +14,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 LIB = os.path.join(PKG, "libbitlattice_b200.so")
+HOST = os.path.join(PKG, "_host.so")                 # host.cpp: Python entry to the library's hot calls
 OBJ = os.path.join(HERE, "_build")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -74,7 +75,33 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if res.returncode:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("linking libbitlattice_b200.so failed")
+    build_host(force, verbose)
     return LIB
+
+
+def build_host(force: bool = False, verbose: bool = False) -> str:
+    """The extension module bitlattice_b200._host (host compiler only; links torch and the library beside it)."""
+    src = os.path.join(HERE, "host.cpp")
+    if not (force or _stale(HOST, [src, os.path.join(os.path.dirname(PKG), "include", "bitlattice_b200.h")])):
+        return HOST
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(os.path.abspath(torch.__file__))
+    nvcc = _nvcc()
+    cuda = os.path.dirname(os.path.dirname(nvcc)) if os.path.sep in nvcc else "/usr/local/cuda"
+    cmd = [os.environ.get("CXX_HOST", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           *[f"-I{d}" for d in (os.path.join(base, "include"), os.path.join(base, "include/torch/csrc/api/include"),
+                                sysconfig.get_paths()["include"], os.path.join(cuda, "include"))],
+           src, "-o", HOST, "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+           "-L" + PKG, "-l:libbitlattice_b200.so", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode:
+        raise RuntimeError("building _host.so failed")
+    return HOST
 
 
 if __name__ == "__main__":

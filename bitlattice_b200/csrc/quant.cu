@@ -329,18 +329,18 @@ __global__ void __launch_bounds__(kQThreads) amax_t_kernel(const T* __restrict__
   if ((threadIdx.x & 31) == 0) atomic_max_pos(out, m);
 }
 
-// global scale of the transposed operand: from a bound (given == 1: in[0] is the bound), from an amax (given == 0),
+// global scale of the transposed operand: from a bound (given == 1: in[0] times factor is the bound), from an amax (given == 0),
 // or as is (given == 2: in[0] already is the scale). The quantizers evaluate it themselves and their first thread
 // publishes it, which saves a launch per operand; the one-thread kernel remains for callers whose output aliases the
 // input.
-__device__ __forceinline__ float global_t(const float* __restrict__ in, int given) {
+__device__ __forceinline__ float global_t(const float* __restrict__ in, int given, float factor) {
   if (given == 2) return in[0];
-  const float amax = given ? in[0] * 2688.0f : in[0];
+  const float amax = given ? in[0] * factor * 2688.0f : in[0];
   return fmaxf(amax / 2688.0f, 1e-12f);
 }
 
-__global__ void global_t_kernel(const float* __restrict__ in, int given, float* __restrict__ global_out) {
-  global_out[0] = global_t(in, given);
+__global__ void global_t_kernel(const float* __restrict__ in, int given, float factor, float* __restrict__ global_out) {
+  global_out[0] = global_t(in, given, factor);
 }
 
 // x [rows, K], read as [M, K] with zeros below -> NVFP4 of x^T. A CTA stages a [128, 64] tile of x in shared memory with coalesced row reads; the work
@@ -348,7 +348,7 @@ __global__ void global_t_kernel(const float* __restrict__ in, int given, float* 
 template <typename T, bool SR>
 __global__ void __launch_bounds__(kQThreads) quantize_t_kernel(const T* __restrict__ x, int64_t rows, int64_t M, int64_t K,
                                                                const float* __restrict__ H,
-                                                               const float* __restrict__ global, int given,
+                                                               const float* __restrict__ global, int given, float factor,
                                                                float* __restrict__ global_out, uint32_t key,
                                                                uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
                                                                int layout) {
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(kQThreads) quantize_t_kernel(const T* __restri
     tile[rr][cc] = (m < rows && k < K) ? to_f<T>(x[m * K + k]) : 0.0f;
   }
   __syncthreads();
-  const float g = global_t(global, given);
+  const float g = global_t(global, given, factor);
   if (global_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) global_out[0] = g;
   // 64 columns x 8 blocks x 2 halves = 1024 work items, 4 per thread; lanes (2j, 2j+1) = halves of one block
   for (int it = 0; it < 4; ++it) {
@@ -444,7 +444,7 @@ __device__ __forceinline__ void rotate16_tree2(const f32x2 p[16], f32x2 v[16]) {
 template <typename T, bool SR>
 __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __restrict__ x, int64_t rows, int64_t M, int64_t K,
                                                                 const float* __restrict__ H,
-                                                                const float* __restrict__ global, int given,
+                                                                const float* __restrict__ global, int given, float factor,
                                                                 float* __restrict__ global_out, uint32_t key,
                                                                 uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
                                                                 int layout) {
@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
         if (m + i < rows) load2(p + i * K, ra[i], rb[i]);
       }
     }
-    const float g = global_t(global, given);
+    const float g = global_t(global, given, factor);
     if (global_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) global_out[0] = g;
     const float rg = __frcp_rn(g);
     f32x2 v2[16];
@@ -937,7 +937,7 @@ extern "C" int bl_nvfp4_quantize_4over6(const void* x, int dtype, int64_t rows, 
 
 template <typename T>
 static int quantize_t_typed(const T* x, int64_t rows, int64_t M, int64_t K, const float* H, int64_t seed, uint32_t step,
-                            const float* bound, float* amax_scratch, uint8_t* codes, uint8_t* scales, float* gout,
+                            const float* bound, float factor, float* amax_scratch, uint8_t* codes, uint8_t* scales, float* gout,
                             int layout, int device, cudaStream_t st) {
   if (bound == nullptr) {
     BL_CUDA(cudaMemsetAsync(amax_scratch, 0, 16, st));
@@ -948,7 +948,7 @@ static int quantize_t_typed(const T* x, int64_t rows, int64_t M, int64_t K, cons
   int given = bound == nullptr ? 0 : 1;
   float* publish = gout;
   if (static_cast<const void*>(gout) == static_cast<const void*>(src)) {     // in-place: settle the scale first
-    global_t_kernel<<<1, 1, 0, st>>>(src, given, gout);
+    global_t_kernel<<<1, 1, 0, st>>>(src, given, factor, gout);
     BL_CUDA(cudaGetLastError());
     src = gout;
     given = 2;
@@ -957,16 +957,16 @@ static int quantize_t_typed(const T* x, int64_t rows, int64_t M, int64_t K, cons
   const dim3 grid(static_cast<unsigned>((K + kTK - 1) / kTK), static_cast<unsigned>((M + kTM - 1) / kTM));
   const uint32_t key = seed < 0 ? 0u : hash_key(static_cast<uint32_t>(seed), step);
   const bool pairs = K % 2 == 0 && (reinterpret_cast<uintptr_t>(x) % (2 * sizeof(T))) == 0;
-  if (pairs && seed < 0) quantize_t3_kernel<T, false><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, publish, key, codes, scales, layout);
-  else if (pairs) quantize_t3_kernel<T, true><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, publish, key, codes, scales, layout);
-  else if (seed < 0) quantize_t_kernel<T, false><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, publish, key, codes, scales, layout);
-  else quantize_t_kernel<T, true><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, publish, key, codes, scales, layout);
+  if (pairs && seed < 0) quantize_t3_kernel<T, false><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, factor, publish, key, codes, scales, layout);
+  else if (pairs) quantize_t3_kernel<T, true><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, factor, publish, key, codes, scales, layout);
+  else if (seed < 0) quantize_t_kernel<T, false><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, factor, publish, key, codes, scales, layout);
+  else quantize_t_kernel<T, true><<<grid, kQThreads, 0, st>>>(x, rows, M, K, H, src, given, factor, publish, key, codes, scales, layout);
   BL_CUDA(cudaGetLastError());
   return 0;
 }
 
 extern "C" int bl_nvfp4_quantize_t_rows(const void* x, int dtype, int64_t rows, int64_t M, int64_t K, const float* H, int64_t seed,
-                                        uint32_t step, const float* global_bound, float* amax_scratch, uint8_t* codes,
+                                        uint32_t step, const float* global_bound, float bound_factor, float* amax_scratch, uint8_t* codes,
                                         uint8_t* scales, float* global_out, int sf_layout, int device, bl_stream_t stream) {
   BL_REQUIRE(x && codes && scales && global_out, "quantize_nvfp4_t: null buffer");
   BL_REQUIRE(M > 0 && K > 0 && M % 16 == 0, "quantize_nvfp4_t: rows must be a multiple of 16, got %lld x %lld",
@@ -983,16 +983,16 @@ extern "C" int bl_nvfp4_quantize_t_rows(const void* x, int dtype, int64_t rows, 
   if (sf_layout == BL_SF_BLOCKED && blocked_needs_padding(K, M / 16))
     BL_CUDA(cudaMemsetAsync(scales, 0, bl_blocked_scale_bytes(K, M / 16), st));
   if (dtype == BL_BF16)
-    return quantize_t_typed(static_cast<const __nv_bfloat16*>(x), rows, M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
+    return quantize_t_typed(static_cast<const __nv_bfloat16*>(x), rows, M, K, H, seed, step, global_bound, bound_factor, amax_scratch, codes, scales, global_out, sf_layout, device, st);
   if (dtype == BL_F16)
-    return quantize_t_typed(static_cast<const __half*>(x), rows, M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
-  return quantize_t_typed(static_cast<const float*>(x), rows, M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out, sf_layout, device, st);
+    return quantize_t_typed(static_cast<const __half*>(x), rows, M, K, H, seed, step, global_bound, bound_factor, amax_scratch, codes, scales, global_out, sf_layout, device, st);
+  return quantize_t_typed(static_cast<const float*>(x), rows, M, K, H, seed, step, global_bound, bound_factor, amax_scratch, codes, scales, global_out, sf_layout, device, st);
 }
 
 extern "C" int bl_nvfp4_quantize_t(const void* x, int dtype, int64_t M, int64_t K, const float* H, int64_t seed,
                                    uint32_t step, const float* global_bound, float* amax_scratch, uint8_t* codes,
                                    uint8_t* scales, float* global_out, int sf_layout, int device, bl_stream_t stream) {
-  return bl_nvfp4_quantize_t_rows(x, dtype, M, M, K, H, seed, step, global_bound, amax_scratch, codes, scales, global_out,
+  return bl_nvfp4_quantize_t_rows(x, dtype, M, M, K, H, seed, step, global_bound, 1.0f, amax_scratch, codes, scales, global_out,
                                   sf_layout, device, stream);
 }
 

@@ -37,7 +37,7 @@ from .. import _ops
 from ..backend import nvtx as _nvtx
 from . import directions as D_
 from ..packing import packed_cols
-from ..tensor import LatticeTensor
+from ..tensor import _no_overrides, LatticeTensor
 
 __all__ = ["DEFAULTS", "DIRECTIONS", "MOMENTA", "ROUNDINGS", "SCALE_RULES", "Lattice", "defer_fused_updates"]
 
@@ -176,6 +176,10 @@ class Lattice(torch.optim.Optimizer):
     # fused backward: the hook runs on the autograd thread that accumulated the gradient
 
     def _on_grad(self, p: torch.Tensor) -> None:
+        with _no_overrides():
+            self._take_grad(p)
+
+    def _take_grad(self, p: torch.Tensor) -> None:
         if p.grad is None or self._defer or _deferred:
             return
         if self.hook_batch > 1:
@@ -323,6 +327,11 @@ class Lattice(torch.optim.Optimizer):
         if closure is not None:
             with torch.enable_grad():
                 loss = closure()
+        with _no_overrides():                      # dozens of attribute reads per parameter: see tensor.py
+            self._step()
+        return loss
+
+    def _step(self) -> None:
         self.check_gemm_status()                   # a failed GEMM of an earlier step: raise before updating further
         self._flush_pending()
         for g in self.param_groups:
@@ -335,7 +344,6 @@ class Lattice(torch.optim.Optimizer):
         self._done.clear()
         self.wait()
         self._watch_gemm_status()
-        return loss
 
     _matrix: dict = {}             # id(parameter) -> whether it counts as a matrix (shape reads of a tensor subclass
                                    # are slow and these run for every parameter of every step)

@@ -50,7 +50,7 @@ from collections import OrderedDict
 import torch
 import torch.distributed as dist
 
-from .tensor import LatticeTensor, wait_for_update
+from .tensor import _PLAIN, _no_overrides, LatticeTensor, wait_for_update
 
 __all__ = ["ColumnParallelFp4Linear", "ColumnParallelLinear", "GatheredWeights", "SharedInputFp4Linears",
            "TokenParallelFp4Linear", "TokenParallelLinear", "column_parallel_linear", "column_parallel_linears",
@@ -337,14 +337,12 @@ class SharedInputFp4Linears(torch.autograd.Function):
     without its collectives): one quantization of the input for all of them, and in the backward the input gradients
     of the projections are summed in the epilogue of their GEMMs (``fp4_dgrad(add_to=)``, the bits of adding the
     tensors in the order of ``weights``) instead of by autograd's accumulation, which costs a pass over the gradient
-    per extra projection."""
+    per extra projection. ``grad``: whether autograd records; if not, no x^T is kept."""
 
     @staticmethod
-    def forward(ctx, x, recipe, *weights):
+    def forward(ctx, x, recipe, grad, *weights):
         from . import backend
-        K = x.shape[-1]
-        M = x.numel() // K
-        if any(ctx.needs_input_grad[2:]):
+        if grad and any(ctx.needs_input_grad[3:]):
             xq, xt = backend._shared(x, recipe, "fwd+t",
                                      lambda: backend._input_operands(x, recipe, site=backend._site(weights[0], "x")))
         else:
@@ -352,11 +350,17 @@ class SharedInputFp4Linears(torch.autograd.Function):
                 backend._flat_rows(x, 16), recipe)), None
         ctx.weights, ctx.recipe, ctx.xt = weights, recipe, xt
         ctx.x_meta = (x.shape, x.dtype)
-        return tuple(backend.fp4_mm(xq, backend.weight_operand(w), x.dtype)[:M].reshape(*x.shape[:-1], w.shape[0])
+        lead = x.shape[:-1]
+        return tuple(backend.fp4_mm(xq, backend.weight_operand(w), x.dtype).reshape(*lead, w.shape[0])
                      for w in weights)
 
     @staticmethod
     def backward(ctx, *gys):
+        with _no_overrides():
+            return SharedInputFp4Linears._gradients(ctx, *gys)
+
+    @staticmethod
+    def _gradients(ctx, *gys):
         from . import backend
         shape, dtype = ctx.x_meta
         M = 1
@@ -378,25 +382,38 @@ class SharedInputFp4Linears(torch.autograd.Function):
             staged.append((g2p, gq))
         gws = []
         for i, (w, st) in enumerate(zip(ctx.weights, staged)):
-            if st is None or not ctx.needs_input_grad[2 + i] or ctx.xt is None:
+            if st is None or not ctx.needs_input_grad[3 + i] or ctx.xt is None:
                 gws.append(None)
                 continue
             gws.append(backend.fp4_wgrad(st[0], st[1], ctx.xt, w, ctx.recipe).to(w.dtype))
         gx = gx_sum.to(dtype).reshape(shape) if gx_sum is not None else None
-        return (gx, None, *gws)
+        return (gx, None, None, *gws)
 
 
 def shared_input_linears(x: torch.Tensor, weights) -> tuple:
     """``F.linear(x, w)`` for every weight. When all of them take the 'fp4_all' route with the NVIDIA-recipe operands
     they run as one function that quantizes the input once and sums their input gradients in the GEMM epilogues."""
     weights = tuple(weights)
-    if len(weights) > 1 and x.is_cuda and all(isinstance(w, LatticeTensor) and w.dim() == 2 for w in weights):
+    if len(weights) > 1 and all(isinstance(w, LatticeTensor) for w in weights):
+        if type(x) in _PLAIN:
+            with _no_overrides():
+                out = _shared_input_fp4(x, weights)
+        else:
+            out = _shared_input_fp4(x, weights)
+        if out is not None:
+            return out
+    return tuple(torch.nn.functional.linear(x, w) for w in weights)
+
+
+def _shared_input_fp4(x: torch.Tensor, weights: tuple):
+    """The outputs of ``shared_input_linears`` by the shared function, or None where the layers do not qualify."""
+    if x.is_cuda and all(w.dim() == 2 for w in weights):
         from .compute_policy import route
         routes = [route(x, w) for w in weights]
         recipe = routes[0][1].nvfp4
         if all(r[0] == "fp4_all" and r[1].nvfp4 == recipe for r in routes) and recipe.packed_exchange:
-            return SharedInputFp4Linears.apply(x, recipe, *weights)
-    return tuple(torch.nn.functional.linear(x, w) for w in weights)
+            return SharedInputFp4Linears.apply(x, recipe, torch.is_grad_enabled(), *weights)
+    return None
 
 
 def _fp4_all_route(x_shard: torch.Tensor, w):

@@ -250,10 +250,12 @@ BL_API int bl_nvfp4_quantize_t(const void* x, int dtype, int64_t M, int64_t K, c
                         const float* global_bound, float* amax_scratch, uint8_t* codes, uint8_t* scales,
                         float* global_out, int sf_layout, int device, bl_stream_t stream);
 
-/* bl_nvfp4_quantize_t of x [rows, K] followed by M - rows rows of zeros (rows <= M, M % 16 == 0), which are not read. */
+/* bl_nvfp4_quantize_t of x [rows, K] followed by M - rows rows of zeros (rows <= M, M % 16 == 0), which are not read;
+ * the bound is *global_bound * bound_factor. */
 BL_API int bl_nvfp4_quantize_t_rows(const void* x, int dtype, int64_t rows, int64_t M, int64_t K, const float* H, int64_t seed,
-                             uint32_t step, const float* global_bound, float* amax_scratch, uint8_t* codes,
-                             uint8_t* scales, float* global_out, int sf_layout, int device, bl_stream_t stream);
+                             uint32_t step, const float* global_bound, float bound_factor, float* amax_scratch,
+                             uint8_t* codes, uint8_t* scales, float* global_out, int sf_layout, int device,
+                             bl_stream_t stream);
 
 /* Replaces torch.ops.bitlattice.requantize_nvfp4_t (csrc/bindings.cpp:99, csrc/act_quant.cu:150-175,273-294):
  * NVFP4 W [N, K] -> NVFP4 of W^T, codes [K, N/2] + scales over [K, N/16], same per-tensor scale (copied to

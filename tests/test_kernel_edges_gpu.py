@@ -213,3 +213,23 @@ def test_ragged_rows_of_a_layer(rows, recipe):
         outs.append((y[:rows], gx[:rows], gw, backend.nvfp4_linear(xi, w, None, recipe)[:rows]))
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("recipe", ["fp4_all", "4over6", "quartet2"])
+def test_outputs_and_draws_do_not_depend_on_grad_mode(recipe):
+    """A forward pass under no_grad makes no operand for the weight gradient: same outputs, single and shared input, and
+    the counter of the rounding seeds moves as it does with gradients."""
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    ps = [torch.nn.Parameter(bl.LatticeTensor.from_float(torch.randn(n, 128, device="cuda", generator=gen) * 0.02, "nvfp4",
+                                                         dtype=torch.bfloat16)) for n in (128, 256)]
+    x = torch.randn(45, 128, device="cuda", generator=gen).to(torch.bfloat16)
+    seen = []
+    for grad in (True, False):
+        backend.set_sr_seed(3)
+        backend.clear_shared()
+        with torch.set_grad_enabled(grad), bl.compute(recipe):
+            ys = (torch.nn.functional.linear(x, ps[0]), *bl.parallel.shared_input_linears(x, ps))
+        assert all(y.requires_grad == grad for y in ys)
+        seen.append((*[y.detach() for y in ys], torch.tensor(backend._seed())))
+    for a, b in zip(*seen):
+        assert torch.equal(a, b)
