@@ -109,6 +109,64 @@ __device__ __forceinline__ uint32_t e4m3_sr(float v, float u) {
   return u < p ? hb : b;
 }
 
+// Nearest codes and scale byte of a block of maximum am, the better of two block scales with four-over-six; t = scale * g.
+__device__ __forceinline__ void nearest_block(const GenArgs& A, const float v[16], float am, float g, uint32_t& sb, float& t,
+                                              float& inv, uint2& codes) {
+  const float rg = __frcp_rn(g);
+  sb = e4m3_encode(div_rn(div_rn(am, 6.0f, 0.16666667163372039794921875f), g, rg));
+  t = e4m3_decode(sb) * g;
+  inv = t > 0.0f ? __frcp_rn(t) : 0.0f;
+  codes = e2m1_nearest16(v, inv);
+  if (A.fos) {
+    const uint32_t sb4 = e4m3_encode(div_rn(am * 0.25f, g, rg));
+    const float t4 = e4m3_decode(sb4) * g;
+    const float inv4 = t4 > 0.0f ? __frcp_rn(t4) : 0.0f;
+    const uint2 codes4 = e2m1_nearest16(v, inv4);
+    const float e6 = candidate_error(v, codes, t, A.mae != 0), e4 = candidate_error(v, codes4, t4, A.mae != 0);
+    if (e4 < e6) {
+      sb = sb4;
+      t = t4;
+      inv = inv4;
+      codes = codes4;
+    }
+  }
+}
+
+// the block's part of <x, x> and <x, x_rtn>
+__device__ __forceinline__ void eden_sums(const float v[16], uint2 codes, float t, float& xx, float& xr) {
+  float d[16];
+  e2m1_levels8(codes.x, d);
+  e2m1_levels8(codes.y, d + 8);
+  float sx[4], sr[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float ax = 0.0f, ar = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      ax = ax + v[4 * q + i] * v[4 * q + i];
+      ar = ar + v[4 * q + i] * (d[4 * q + i] * t);
+    }
+    sx[q] = ax;
+    sr[q] = ar;
+  }
+  xx = (sx[0] + sx[1]) + (sx[2] + sx[3]);
+  xr = (sr[0] + sr[1]) + (sr[2] + sr[3]);
+}
+
+// the scale byte times xx / xr (sums over the 128), rounded stochastically; c16: block of the output row
+__device__ __forceinline__ uint32_t eden_scale(const GenArgs& A, uint32_t sb, float xx, float xr, int64_t r, int64_t c16) {
+  const float S = xr != 0.0f ? xx / xr : 1.0f;
+  const uint32_t block = static_cast<uint32_t>(static_cast<uint64_t>(r) * static_cast<uint64_t>(A.cols / 16) +
+                                               static_cast<uint64_t>(c16));
+  return e4m3_sr(e4m3_decode(sb) * S, hash_uniform(block, A.eden_key));
+}
+
+__device__ __forceinline__ int64_t general_scale_index(const GenArgs& A, int64_t r, int64_t c16) {
+  const int64_t cols16 = A.cols / 16;
+  if (A.layout == BL_SF_ROWMAJOR) return r * cols16 + c16;
+  return ((r >> 7) * ((cols16 + 3) >> 2) + (c16 >> 2)) * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4 + (c16 & 3);
+}
+
 // PASS 0: max |value| of the (rotated) output into A.amax[0] (zeroed by the host). PASS 1: codes and scales.
 // A warp works on four output rows at a time: lanes 8c .. 8c + 7 hold the eight 16-element blocks of row c's segment.
 template <typename T, int SRC, int PASS>
@@ -227,65 +285,29 @@ __global__ void __launch_bounds__(kGenThreads) general_kernel(GenArgs A) {
       wmax = fmaxf(wmax, am);
     } else {
       if (observe) wmax = fmaxf(wmax, am);
-      uint32_t sb = e4m3_encode(am / 6.0f / g);
-      float t = e4m3_decode(sb) * g;
-      float inv = t > 0.0f ? 1.0f / t : 0.0f;
-      uint2 codes = e2m1_nearest16(v, inv);
-      if (A.fos) {
-        const uint32_t sb4 = e4m3_encode(am / 4.0f / g);
-        const float t4 = e4m3_decode(sb4) * g;
-        const float inv4 = t4 > 0.0f ? 1.0f / t4 : 0.0f;
-        const uint2 codes4 = e2m1_nearest16(v, inv4);
-        const float e6 = candidate_error(v, codes, t, A.mae != 0), e4 = candidate_error(v, codes4, t4, A.mae != 0);
-        if (e4 < e6) {
-          sb = sb4;
-          t = t4;
-          inv = inv4;
-          codes = codes4;
-        }
-      }
+      uint32_t sb;
+      float t, inv;
+      uint2 codes;
+      nearest_block(A, v, am, g, sb, t, inv, codes);
       if (A.mode == BL_Q_SR) {
         const uint32_t idx0 = static_cast<uint32_t>(static_cast<uint64_t>(r) * static_cast<uint64_t>(A.cols) +
                                                     static_cast<uint64_t>(col0 + 16 * blk));
         codes = e2m1_sr16(v, inv, A.key, idx0);
       } else if (A.mode == BL_Q_EDEN) {
-        float d[16];
-        e2m1_levels8(codes.x, d);
-        e2m1_levels8(codes.y, d + 8);
-        float sx[4], sr[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float ax = 0.0f, ar = 0.0f;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            ax = ax + v[4 * q + i] * v[4 * q + i];
-            ar = ar + v[4 * q + i] * (d[4 * q + i] * t);
-          }
-          sx[q] = ax;
-          sr[q] = ar;
-        }
-        float xx = (sx[0] + sx[1]) + (sx[2] + sx[3]), xr = (sr[0] + sr[1]) + (sr[2] + sr[3]);
+        float xx, xr;
+        eden_sums(v, codes, t, xx, xr);
 #pragma unroll
         for (int m = 1; m < 8; m <<= 1) {
           xx = xx + __shfl_xor_sync(0xffffffffu, xx, m);
           xr = xr + __shfl_xor_sync(0xffffffffu, xr, m);
         }
-        const float S = xr != 0.0f ? xx / xr : 1.0f;
-        const uint32_t block = static_cast<uint32_t>(static_cast<uint64_t>(r) * static_cast<uint64_t>(A.cols / 16) +
-                                                     static_cast<uint64_t>((col0 + 16 * blk) / 16));
-        sb = e4m3_sr(e4m3_decode(sb) * S, hash_uniform(block, A.eden_key));
+        sb = eden_scale(A, sb, xx, xr, r, col0 / 16 + blk);
       }
       if (valid) {
         codes.x = e2m1_drop_negative_zero(codes.x);
         codes.y = e2m1_drop_negative_zero(codes.y);
         *reinterpret_cast<uint2*>(A.codes + r * (A.cols / 2) + (col0 + 16 * blk) / 2) = codes;
-        const int64_t c16 = (col0 + 16 * blk) / 16, cols16 = A.cols / 16;
-        int64_t at = r * cols16 + c16;
-        if (A.layout != BL_SF_ROWMAJOR) {
-          const int64_t nc = (cols16 + 3) >> 2;
-          at = ((r >> 7) * nc + (c16 >> 2)) * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4 + (c16 & 3);
-        }
-        A.scales[at] = static_cast<uint8_t>(sb);
+        A.scales[general_scale_index(A, r, col0 / 16 + blk)] = static_cast<uint8_t>(sb);
       }
     }
   }
@@ -294,6 +316,262 @@ __global__ void __launch_bounds__(kGenThreads) general_kernel(GenArgs A) {
     for (int o = 16; o > 0; o >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
     if (lane == 0 && wmax > 0.0f) atomicMax(reinterpret_cast<int*>(PASS == 0 ? A.amax : A.amax_out), __float_as_int(wmax));
   }
+}
+
+// ---- rotated operands: two output rows at a time in packed pairs --------------------------------------------------------
+// What bounded general_kernel on them was the rotation: 4 additions, 3 shuffles and 3 multiply-adds per element one row at a
+// time, 16 sign hashes per lane for 32 elements, and for transposed output a staged tile whose reads met 4-way bank
+// conflicts. Here the two lanes of packed fp32 arithmetic are two output rows, the signs are hashed once for 256 rows, a
+// transposed tile is read straight into registers, and the strides across blocks go through shared memory once (1.5
+// additions an element) instead of by shuffles. Same butterflies in the same order: the same bits. 16384 x 4096 bf16,
+// MS-EDEN, maximum and quantization pass: transposed 93 -> 44 and 130 -> 101 us, rows 65 -> 56 and 116 -> 108 us; 4096 x 4096 from
+// NVFP4 27 -> 17 and 38 -> 35 us.
+
+constexpr int kRotTiles = 4;        // tiles of 64 output rows of a CTA
+
+// eden_sums of two blocks, one in each lane of the pairs
+__device__ __forceinline__ void eden_sums2(const f32x2 v[16], const uint2 codes[2], const float t[2], float2& xx, float2& xr) {
+  float da[16], db[16];
+  e2m1_levels8(codes[0].x, da);
+  e2m1_levels8(codes[0].y, da + 8);
+  e2m1_levels8(codes[1].x, db);
+  e2m1_levels8(codes[1].y, db + 8);
+  const f32x2 t2 = pk(t[0], t[1]);
+  f32x2 sx[4], sr[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    f32x2 ax = pk(0.0f, 0.0f), ar = pk(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 4 * q; i < 4 * q + 4; ++i) {
+      ax = add2p(ax, prod2p(v[i], v[i]));
+      ar = add2p(ar, prod2p(v[i], mul2p(pk(da[i], db[i]), t2)));
+    }
+    sx[q] = ax;
+    sr[q] = ar;
+  }
+  upk(add2p(add2p(sx[0], sx[1]), add2p(sx[2], sx[3])), xx.x, xx.y);
+  upk(add2p(add2p(sr[0], sr[1]), add2p(sr[2], sr[3])), xr.x, xr.y);
+}
+
+// bit i: the rotation negates element 16 blk + i of its segment
+__device__ __forceinline__ uint32_t rotation_signs(const GenArgs& A, int blk) {
+  uint32_t neg = 0;
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    neg |= (hash_uniform(static_cast<uint32_t>(16 * blk + i), A.rot_key) < 0.5f ? 1u : 0u) << i;
+  return neg;
+}
+
+__device__ __forceinline__ void butterflies16(f32x2 v[16]) {                         // strides 1 .. 8
+#pragma unroll
+  for (int h = 1; h < 16; h <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if ((i & h) == 0) {
+        const f32x2 a = v[i], b = v[i + h];
+        v[i] = add2p(a, b);
+        v[i + h] = sub2p(a, b);
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void split16(const f32x2 v[16], float a[16], float b[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) upk(v[i], a[i], b[i]);
+}
+
+__device__ __forceinline__ void publish_max(float wmax, float* out) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
+  if ((threadIdx.x & 31) == 0 && wmax > 0.0f) atomicMax(reinterpret_cast<int*>(out), __float_as_int(wmax));
+}
+
+__device__ __forceinline__ float publish_global(const GenArgs& A) {
+  const float g = general_global(A);
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    A.out_global[0] = g;
+    if (A.amax_out && !A.given) A.amax_out[0] = A.amax[0];
+  }
+  return g;
+}
+
+// A tile is 64 output rows, as 32 pairs (slots). Loading: for transposed output warp b reads block b of the segment --
+// source rows col0 + 16 b .. + 15 -- and lane l the source columns 2 l and 2 l + 1 (an even number of them exists), one word
+// a row; for output rows that are source rows, lanes 8 c .. 8 c + 7 of warp w read the eight blocks of rows 8 w + c and
+// 8 w + c + 4. After strides 1 .. 8 every thread leaves its 16 pairs in shared memory, [block][position][slot] (the padding
+// keeps both ways of loading free of conflicts); thread (b, l) takes the eight blocks' pairs of positions 2 b and 2 b + 1 of
+// slot l through strides 16 .. 64, puts them back and, in pass 1, collects the 16 of block b to quantize.
+template <typename T, int SRC, int PASS>
+__global__ void __launch_bounds__(kGenThreads, 3) rotated_kernel(GenArgs A) {
+  __shared__ f32x2 ex[8][16 * 32 + 4];
+  __shared__ float2 s_sums[PASS == 1 ? 2 : 1][8][32];
+  __shared__ uint2 s_codes[PASS == 1 ? kGenTileRows : 1][8 + 1];
+  __shared__ __align__(8) uint8_t s_scales[PASS == 1 ? kGenTileRows : 1][8];
+  const bool words = (reinterpret_cast<uintptr_t>(A.scales) & 3u) == 0;
+  const int b = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int64_t col0 = static_cast<int64_t>(blockIdx.x) * 128;
+  const int load_blk = SRC == kSrcRows ? l & 7 : b, load_slot = SRC == kSrcRows ? 4 * b + (l >> 3) : l;
+  const uint32_t neg = rotation_signs(A, load_blk);
+  const float g = PASS == 1 ? publish_global(A) : 1.0f;
+  const bool observe = PASS == 1 && A.amax_out && A.given;
+  float wmax = 0.0f;
+  for (int tile = 0; tile < kRotTiles; ++tile) {
+    const int64_t row0 = (static_cast<int64_t>(blockIdx.y) * kRotTiles + tile) * kGenTileRows;
+    if (row0 >= A.rows) break;                             // the same for the whole CTA
+    f32x2 v[16];
+    if constexpr (SRC == kSrcRows) {
+      const int64_t r = row0 + 8 * b + (l >> 3);
+      const T* x = static_cast<const T*>(A.x) + r * A.C + col0 + 16 * load_blk;
+      float va[16], vb[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) va[i] = vb[i] = 0.0f;
+      if (r < A.rows) {
+        load8(x, va);
+        load8(x + 8, va + 8);
+      }
+      if (r + 4 < A.rows) {
+        load8(x + 4 * A.C, vb);
+        load8(x + 4 * A.C + 8, vb + 8);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = pk(va[i], vb[i]);
+    } else if (const int64_t r = row0 + 2 * l; r < A.rows) {
+      if constexpr (SRC == kSrcTransposed) {
+        const T* x = static_cast<const T*>(A.x) + (col0 + 16 * b) * A.C + r;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float lo, hi;
+          if constexpr (sizeof(T) == 2) {
+            const uint32_t w = *reinterpret_cast<const uint32_t*>(x + i * A.C);
+            const T* e = reinterpret_cast<const T*>(&w);
+            lo = to_f<T>(e[0]);
+            hi = to_f<T>(e[1]);
+          } else {
+            const float2 w = *reinterpret_cast<const float2*>(x + i * A.C);
+            lo = w.x;
+            hi = w.y;
+          }
+          v[i] = pk(lo, hi);
+        }
+      } else {
+        const uint8_t* codes = static_cast<const uint8_t*>(A.x) + (col0 + 16 * b) * (A.C / 2) + r / 2;
+        const uint8_t* scales = A.w_scales + (col0 + 16 * b) * (A.C / 16) + r / 16;
+        const float gw = A.w_global[0];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          uint32_t h2;
+          asm("{\n\t.reg .b8 b;\n\tcvt.u8.u32 b, %1;\n\tcvt.rn.f16x2.e2m1x2 %0, b;\n\t}" : "=r"(h2) : "r"(static_cast<uint32_t>(codes[i * (A.C / 2)])));
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h2));
+          const float s = e4m3_decode(scales[i * (A.C / 16)]);
+          v[i] = pk((f.x * s) * gw, (f.y * s) * gw);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = pk(0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float lo, hi;
+      upk(v[i], lo, hi);
+      const uint32_t m = (neg << (31 - i)) & 0x80000000u;
+      v[i] = pk(__uint_as_float(__float_as_uint(lo) ^ m), __uint_as_float(__float_as_uint(hi) ^ m));
+    }
+    butterflies16(v);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) ex[load_blk][i * 32 + load_slot] = v[i];
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int i = 2 * b + e;
+      f32x2 w[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w[k] = ex[k][i * 32 + l];
+#pragma unroll
+      for (int h = 1; h < 8; h <<= 1) {                                              // strides 16 .. 64
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if ((k & h) == 0) {
+            const f32x2 p = w[k], q = w[k + h];
+            w[k] = add2p(p, q);
+            w[k + h] = sub2p(p, q);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w[k] = mul2p(w[k], pk(kInvSqrt128, kInvSqrt128));
+      if constexpr (PASS == 0) {
+        float p[16];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) upk(w[k], p[2 * k], p[2 * k + 1]);
+        wmax = fmaxf(wmax, max_abs16(p));
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ex[k][i * 32 + l] = w[k];
+      }
+    }
+    __syncthreads();
+    if constexpr (PASS == 1) {
+      const int pair[2] = {SRC == kSrcRows ? 8 * (l >> 2) + (l & 3) : 2 * l, SRC == kSrcRows ? 8 * (l >> 2) + (l & 3) + 4 : 2 * l + 1};
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = ex[b][i * 32 + l];
+      float va[16], vb[16];
+      split16(v, va, vb);
+      const float am[2] = {max_abs16(va), max_abs16(vb)};
+      if (observe) wmax = fmaxf(wmax, fmaxf(am[0], am[1]));
+      uint32_t sb[2];
+      float t[2], inv[2];
+      uint2 codes[2];
+      nearest_block(A, va, am[0], g, sb[0], t[0], inv[0], codes[0]);
+      nearest_block(A, vb, am[1], g, sb[1], t[1], inv[1], codes[1]);
+      if (A.mode == BL_Q_SR) {
+        const uint32_t idx = static_cast<uint32_t>(static_cast<uint64_t>(row0) * static_cast<uint64_t>(A.cols) +
+                                                   static_cast<uint64_t>(col0 + 16 * b));
+        codes[0] = e2m1_sr16(va, inv[0], A.key, idx + static_cast<uint32_t>(pair[0]) * static_cast<uint32_t>(A.cols));
+        codes[1] = e2m1_sr16(vb, inv[1], A.key, idx + static_cast<uint32_t>(pair[1]) * static_cast<uint32_t>(A.cols));
+      } else if (A.mode == BL_Q_EDEN) {
+        float2 xx, xr;
+        eden_sums2(v, codes, t, xx, xr);
+        s_sums[0][b][l] = xx;
+        s_sums[1][b][l] = xr;
+        __syncthreads();
+        float2 sum[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float2 p[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) p[k] = s_sums[q][k][l];
+          sum[q].x = ((p[0].x + p[1].x) + (p[2].x + p[3].x)) + ((p[4].x + p[5].x) + (p[6].x + p[7].x));
+          sum[q].y = ((p[0].y + p[1].y) + (p[2].y + p[3].y)) + ((p[4].y + p[5].y) + (p[6].y + p[7].y));
+        }
+        sb[0] = eden_scale(A, sb[0], sum[0].x, sum[1].x, row0 + pair[0], col0 / 16 + b);
+        sb[1] = eden_scale(A, sb[1], sum[0].y, sum[1].y, row0 + pair[1], col0 / 16 + b);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        s_codes[pair[e]][b] = make_uint2(e2m1_drop_negative_zero(codes[e].x), e2m1_drop_negative_zero(codes[e].y));
+        s_scales[pair[e]][b] = static_cast<uint8_t>(sb[e]);
+      }
+      __syncthreads();
+      // write-out: thread -> (row of the tile, two of its eight blocks)
+      const int row = threadIdx.x >> 2, b0 = (threadIdx.x & 3) * 2;
+      if (row0 + row < A.rows) {
+        const uint2 lo = s_codes[row][b0], hi = s_codes[row][b0 + 1];
+        *reinterpret_cast<uint4*>(A.codes + (row0 + row) * (A.cols / 2) + col0 / 2 + 8 * b0) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        // four neighbouring scales of a row are one word in either layout
+        uint8_t* dst = A.scales + general_scale_index(A, row0 + row, col0 / 16 + b0);
+        if (words) {
+          if ((b0 & 2) == 0) *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(&s_scales[row][b0]);
+        } else {
+          dst[0] = s_scales[row][b0];
+          dst[1] = s_scales[row][b0 + 1];
+        }
+      }
+      // (the next tile's first barrier stands between these reads and its writes of s_codes, s_scales and s_sums)
+    }
+  }
+  if (PASS == 0 || observe) publish_max(wmax, PASS == 0 ? A.amax : A.amax_out);
 }
 
 // Scales of deferred weight-gradient operands brought to a common per-tensor scale: piece j (one micro-batch) has the
@@ -322,11 +600,52 @@ __global__ void __launch_bounds__(256) fold_scales_kernel(uint8_t* __restrict__ 
   if ((threadIdx.x & 31) == 0 && count) atomicAdd(rounded, count);
 }
 
+// max |x| without the rotation: a plain pass over the source (16-byte loads; n is a multiple of 16). 16384 x 4096 bf16: 56 ->
+// 32 us against the general kernel's pass 0.
 template <typename T>
-static int general_typed(GenArgs A, bool packed, bool transpose, bool need_amax, cudaStream_t st) {
+__global__ void __launch_bounds__(kGenThreads) general_amax_kernel(const T* __restrict__ x, int64_t n, float* __restrict__ amax) {
+  constexpr int kPer = 16 / sizeof(T);
+  float m = 0.0f;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n / kPer;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const uint4 raw = reinterpret_cast<const uint4*>(x)[i];
+    const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) m = fmaxf(m, fabsf(to_f<T>(e[j])));
+  }
+  publish_max(m, amax);
+}
+
+template <typename T>
+static int general_typed(GenArgs A, bool packed, bool transpose, bool need_amax, int device, cudaStream_t st) {
   const dim3 grid(static_cast<unsigned>((A.cols + 127) / 128), static_cast<unsigned>((A.rows + kGenTileRows - 1) / kGenTileRows));
+  if (need_amax) BL_CUDA(cudaMemsetAsync(A.amax, 0, sizeof(float), st));
+  // Rotated operands (cols is a multiple of 128): two rows at a time. Transposed ones read pairs of source columns, so
+  // their number must be even and the source aligned to a pair.
+  if (A.rotate && (!transpose || (A.rows % 2 == 0 && reinterpret_cast<uintptr_t>(A.x) % (2 * sizeof(T)) == 0))) {
+    constexpr unsigned kPer = kRotTiles * kGenTileRows;
+    const dim3 rot(grid.x, static_cast<unsigned>((A.rows + kPer - 1) / kPer));
+    for (int pass = need_amax ? 0 : 1; pass < 2; ++pass) {
+      if (packed) {
+        if (pass == 0) rotated_kernel<uint8_t, kSrcPackedTransposed, 0><<<rot, kGenThreads, 0, st>>>(A);
+        else rotated_kernel<uint8_t, kSrcPackedTransposed, 1><<<rot, kGenThreads, 0, st>>>(A);
+      } else if (transpose) {
+        if (pass == 0) rotated_kernel<T, kSrcTransposed, 0><<<rot, kGenThreads, 0, st>>>(A);
+        else rotated_kernel<T, kSrcTransposed, 1><<<rot, kGenThreads, 0, st>>>(A);
+      } else {
+        if (pass == 0) rotated_kernel<T, kSrcRows, 0><<<rot, kGenThreads, 0, st>>>(A);
+        else rotated_kernel<T, kSrcRows, 1><<<rot, kGenThreads, 0, st>>>(A);
+      }
+      BL_CUDA(cudaGetLastError());
+    }
+    return 0;
+  }
+  if (need_amax && !A.rotate && !packed) {
+    const int64_t n = A.R * A.C, want = (n * sizeof(T) / 16 + kGenThreads - 1) / kGenThreads, most = static_cast<int64_t>(sm_count(device)) * 16;
+    general_amax_kernel<T><<<static_cast<unsigned>(want < most ? want : most), kGenThreads, 0, st>>>(static_cast<const T*>(A.x), n, A.amax);
+    need_amax = false;
+  }
   if (need_amax) {
-    BL_CUDA(cudaMemsetAsync(A.amax, 0, sizeof(float), st));
     if (packed) general_kernel<uint8_t, kSrcPackedTransposed, 0><<<grid, kGenThreads, 0, st>>>(A);
     else if (transpose) general_kernel<T, kSrcTransposed, 0><<<grid, kGenThreads, 0, st>>>(A);
     else general_kernel<T, kSrcRows, 0><<<grid, kGenThreads, 0, st>>>(A);
@@ -398,9 +717,9 @@ extern "C" int bl_nvfp4_quantize_general(const void* x, int dtype, int64_t R, in
     BL_CUDA(cudaMemsetAsync(scales, 0, bl_blocked_scale_bytes(rows, cols / 16), st));
   const bool need_amax = given_global == nullptr;
   if (amax_out && !need_amax) BL_CUDA(cudaMemsetAsync(amax_out, 0, sizeof(float), st));
-  if (packed || dtype == BL_BF16) return general_typed<__nv_bfloat16>(A, packed, transpose != 0, need_amax, st);
-  if (dtype == BL_F16) return general_typed<__half>(A, packed, transpose != 0, need_amax, st);
-  return general_typed<float>(A, packed, transpose != 0, need_amax, st);
+  if (packed || dtype == BL_BF16) return general_typed<__nv_bfloat16>(A, packed, transpose != 0, need_amax, device, st);
+  if (dtype == BL_F16) return general_typed<__half>(A, packed, transpose != 0, need_amax, device, st);
+  return general_typed<float>(A, packed, transpose != 0, need_amax, device, st);
 }
 
 extern "C" int bl_fp4_fold_scales(uint8_t* scales, int64_t row_tiles, int64_t tiles_per_row, const int* piece,

@@ -164,3 +164,20 @@ def test_fold_scales_matches_oracle():
             count += n
     assert np.array_equal(host(dev_sc).reshape(row_tiles, tiles_per_row, 512), want)
     assert int(rounded.item()) == count and count > 0
+
+
+@pytest.mark.parametrize("shape,transpose", [((1, 128), False), ((5, 256), False), ((261, 128), False), ((128, 2), True),
+                                             ((256, 66), True), ((128, 322), True), ((128, 7), True)])
+@pytest.mark.parametrize("mode,fos", [("rtn", True), ("sr", False), ("eden", False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_ragged_shapes_with_rotation(shape, transpose, mode, fos, dtype):
+    """Rotated operands whose rows end inside a CTA's rows, inside a tile of 64 and after a single pair; an odd number of
+    transposed rows, which takes the general kernel: against the oracle, blocked and row-major scales."""
+    x = torch.randn(*shape, generator=torch.Generator().manual_seed(sum(shape))).to(dtype)
+    kw = dict(transpose=transpose, mode=mode, four_over_six=fos, rotate=True, seed=3, rotate_seed=8)
+    codes, osb, og = G.quantize(x.float().numpy(), **kw)
+    packed, sb, g = run(x.to(DEV), **kw)
+    assert g == float(og) and np.array_equal(sb, osb) and np.array_equal(packed, G.pack(codes))
+    import oracle
+    packed, sb, g = run(x.to(DEV), blocked=True, **kw)
+    assert np.array_equal(packed, G.pack(codes)) and np.array_equal(sb.reshape(-1), oracle.to_blocked(osb).reshape(-1))
