@@ -233,3 +233,23 @@ def test_outputs_and_draws_do_not_depend_on_grad_mode(recipe):
         seen.append((*[y.detach() for y in ys], torch.tensor(backend._seed())))
     for a, b in zip(*seen):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 16), (3, 48), (16, 4096), (129, 80), (1, 262144), (64, 4096), (257, 1024), (64, 4112)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("seed", [-1, 9])
+def test_amax_quantize_small_and_separate(rows, cols, dtype, seed):
+    """Maximum and quantization in one launch (up to 262144 values, and just above) against the two operators: codes, every
+    scale byte of the tiles, padding included, and the four results of the maximum but its counter."""
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = (torch.randn(rows, cols, device="cuda", generator=gen) * 3).to(dtype)
+    x[-1, -1] = 40.0
+    if rows > 100:
+        x[0] = 0.0
+    am = _ops.amax_global(x)
+    for blocked in (True, False):
+        codes, scales = _ops.quantize_nvfp4(x, am[1:2], seed, 2, blocked=blocked)
+        torch.full((1 << 20,), 0x7F, dtype=torch.uint8, device="cuda")             # stale bytes for the next allocations
+        c, s, a = _ops.amax_quantize_nvfp4(x, seed, 2, blocked=blocked)
+        assert torch.equal(c, codes) and torch.equal(s.view(torch.uint8), scales.view(torch.uint8))
+        assert torch.equal(a[[0, 1, 3]], am[[0, 1, 3]])
