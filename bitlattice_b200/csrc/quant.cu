@@ -22,19 +22,41 @@ __device__ __forceinline__ void atomic_max_pos(float* addr, float v) {   // v >=
   atomicMax(reinterpret_cast<int*>(addr), __float_as_int(v));
 }
 
+// max |element| of 16 bytes; 16-bit types two at a time, without unpacking
+template <typename T>
+__device__ __forceinline__ float max_abs_vec(const uint4& r) {
+  if constexpr (sizeof(T) == 4) {
+    return max_abs3(max_abs3(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z)), __uint_as_float(r.w), 0.0f);
+  } else {
+    using T2 = typename std::conditional<std::is_same<T, __nv_bfloat16>::value, __nv_bfloat162, __half2>::type;
+    const T2* w = reinterpret_cast<const T2*>(&r);
+    const T2 m = __hmax2(__hmax2(__habs2(w[0]), __habs2(w[1])), __hmax2(__habs2(w[2]), __habs2(w[3])));
+    return fmaxf(to_f<T>(m.x), to_f<T>(m.y));
+  }
+}
+
 // out[0] = max|x| (out must start at zero); the last block to finish writes out[1] = max(out[0] / 2688, 1e-12) and
 // out[3] = max(out[0] / 1536, 1e-12); out[2] is the ticket counter
-template <typename T>
+template <typename T, int kAmaxLoads>
 __global__ void __launch_bounds__(kQThreads) amax_kernel(const T* __restrict__ x, int64_t n, float* __restrict__ out) {
   constexpr int per = 16 / sizeof(T);
   const int64_t nvec = n / per;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   float m = 0.0f;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint4 raw = reinterpret_cast<const uint4*>(x)[i];
-    const T* e = reinterpret_cast<const T*>(&raw);
+  int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (; i + (kAmaxLoads - 1) * stride < nvec; i += kAmaxLoads * stride) {
+    uint4 raw[kAmaxLoads];
 #pragma unroll
-    for (int j = 0; j < per; ++j) m = fmaxf(m, fabsf(to_f<T>(e[j])));
+    for (int q = 0; q < kAmaxLoads; ++q) raw[q] = reinterpret_cast<const uint4*>(x)[i + q * stride];
+#pragma unroll
+    for (int q = 0; q < kAmaxLoads; ++q) m = fmaxf(m, max_abs_vec<T>(raw[q]));
+  }
+  {                                                        // fewer than kAmaxLoads vectors left: together as well
+    uint4 raw[kAmaxLoads];
+#pragma unroll
+    for (int q = 0; q < kAmaxLoads; ++q) raw[q] = i + q * stride < nvec ? reinterpret_cast<const uint4*>(x)[i + q * stride] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int q = 0; q < kAmaxLoads; ++q) m = fmaxf(m, max_abs_vec<T>(raw[q]));
   }
   if (blockIdx.x == 0 && threadIdx.x < n - nvec * per) m = fmaxf(m, fabsf(to_f<T>(x[nvec * per + threadIdx.x])));
 #pragma unroll
@@ -935,11 +957,21 @@ extern "C" int bl_nvfp4_amax(const void* x, int dtype, int64_t n, float* out, in
   BL_DEVICE(device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   BL_CUDA(cudaMemsetAsync(out, 0, 16, st));
-  const int per = dtype == BL_F32 ? 4 : 8;
-  const int grid = grid_for(n / per + 1, kQThreads, device);
-  if (dtype == BL_BF16) amax_kernel<<<grid, kQThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(x), n, out);
-  else if (dtype == BL_F16) amax_kernel<<<grid, kQThreads, 0, st>>>(static_cast<const __half*>(x), n, out);
-  else amax_kernel<<<grid, kQThreads, 0, st>>>(static_cast<const float*>(x), n, out);
+  // Four CTAs per SM with eight loads in flight per thread keep 128 KB under way on each and leave a quarter of the atomics
+  // at the end: 1903 x 4096 bf16 6.8 -> 4.6 us, 4096 x 4096 8.0 -> 5.7 us, 4999 x 25600 fp16 40.3 -> 38.9 us. From 256 MB on
+  // the end no longer counts and sixteen CTAs of single loads are 2 to 3 % ahead (65536 x 4096: 78 against 80 us).
+  const int64_t vecs = n / (dtype == BL_F32 ? 4 : 8) + 1;
+  const bool large = vecs >= (int64_t(1) << 24);
+  const int64_t wave = static_cast<int64_t>(sm_count(device)) * (large ? 16 : 4), want = (vecs + kQThreads - 1) / kQThreads;
+  const int grid = static_cast<int>(want < wave ? want : wave);
+  auto launch = [&](auto* p) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
+    if (large) amax_kernel<T, 1><<<grid, kQThreads, 0, st>>>(p, n, out);
+    else amax_kernel<T, 8><<<grid, kQThreads, 0, st>>>(p, n, out);
+  };
+  if (dtype == BL_BF16) launch(static_cast<const __nv_bfloat16*>(x));
+  else if (dtype == BL_F16) launch(static_cast<const __half*>(x));
+  else launch(static_cast<const float*>(x));
   BL_CUDA(cudaGetLastError());
   return 0;
 }

@@ -253,3 +253,19 @@ def test_amax_quantize_small_and_separate(rows, cols, dtype, seed):
         c, s, a = _ops.amax_quantize_nvfp4(x, seed, 2, blocked=blocked)
         assert torch.equal(c, codes) and torch.equal(s.view(torch.uint8), scales.view(torch.uint8))
         assert torch.equal(a[[0, 1, 3]], am[[0, 1, 3]])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n", [1, 7, 4099, 148 * 4 * 256 * 8 * 8 + 5, (1 << 27) + 9])
+def test_amax_finds_every_position(n, dtype):
+    """The maximum at the first, a middle and the last element (whole rounds of loads, the last partial round, the ragged
+    tail, the grid of large tensors), a NaN ignored as before, an infinity found."""
+    x = torch.full((n,), -0.5, dtype=dtype, device="cuda")
+    for at in sorted({0, n // 2, max(0, n - 9), n - 1}):
+        x[at] = -3.0
+        assert _ops.amax_global(x)[0].item() == 3.0
+        x[at] = -0.5
+    x[n // 3] = float("nan")
+    assert _ops.amax_global(x)[0].item() == (0.5 if n > 1 else 0.0)
+    x[n // 3] = float("inf")
+    assert _ops.amax_global(x)[0].item() == float("inf")
