@@ -9,7 +9,8 @@
 //   4/6 error  per block: sequential sums over elements 4q .. 4q + 3, then (s0 + s1) + (s2 + s3)
 //   MS-EDEN    <x, x> and <x, x_rtn> per 128: sequential sums over 4 elements, then a pairwise tree (neighbours first)
 //
-// Thread mapping: a lane owns one 16-element block, eight neighbouring lanes one 128-element segment of an output row,
+// Thread mapping of general_kernel (unrotated operands; rotated_kernel below takes the others but an odd number of
+// transposed rows): a lane owns one 16-element block, eight neighbouring lanes one 128-element segment of an output row,
 // a warp four rows' segments at a time. Strides 1 .. 8 of the rotation run in registers, strides 16 .. 64 are shuffles
 // over lane distances 1, 2, 4; block scales, four-over-six errors and stochastic draws need no exchange, the MS-EDEN
 // sums three shuffle steps. A CTA covers 128 output columns x 64 output rows; for transposed output it first stages
