@@ -337,7 +337,11 @@ class SharedInputFp4Linears(torch.autograd.Function):
     without its collectives): one quantization of the input for all of them, and in the backward the input gradients
     of the projections are summed in the epilogue of their GEMMs (``fp4_dgrad(add_to=)``, the bits of adding the
     tensors in the order of ``weights``) instead of by autograd's accumulation, which costs a pass over the gradient
-    per extra projection. ``grad``: whether autograd records; if not, no x^T is kept."""
+    per extra projection. If autograd does not record, no x^T is kept."""
+
+    @classmethod
+    def apply(cls, x, recipe, *weights):
+        return super().apply(x, recipe, torch.is_grad_enabled(), *weights)      # forward itself always runs without it
 
     @staticmethod
     def forward(ctx, x, recipe, grad, *weights):
@@ -412,7 +416,7 @@ def _shared_input_fp4(x: torch.Tensor, weights: tuple):
         routes = [route(x, w) for w in weights]
         recipe = routes[0][1].nvfp4
         if all(r[0] == "fp4_all" and r[1].nvfp4 == recipe for r in routes) and recipe.packed_exchange:
-            return SharedInputFp4Linears.apply(x, recipe, torch.is_grad_enabled(), *weights)
+            return SharedInputFp4Linears.apply(x, recipe, *weights)
     return None
 
 
