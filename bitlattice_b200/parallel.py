@@ -603,18 +603,16 @@ class TokenParallelFp4Linear(torch.autograd.Function):
     def forward(ctx, x, gathered, recipe, *weights):
         from . import backend
         need_w = any(ctx.needs_input_grad[3:])
-        K = x.shape[-1]
-        M = x.numel() // K
         if need_w:
             xq, xt = backend._shared(x, recipe, "fwd+t", lambda: backend._input_operands(x, recipe))
         else:
-            xq = backend._shared(x, recipe, "fwd", lambda: backend._act_operand(
-                backend._pad_rows(x.reshape(-1, K), 16).contiguous(), recipe))
+            # (the rows there are: the plain layers keep the same operand under the same key and do not cut the product)
+            xq = backend._shared(x, recipe, "fwd", lambda: backend._act_operand(backend._flat_rows(x, 16), recipe))
             xt = None
         ctx.gathered, ctx.weights, ctx.recipe, ctx.xt = gathered, weights, recipe, xt
         ctx.x_meta = (x.shape, x.dtype)
         size = world(gathered.group)[1]
-        return tuple(backend.fp4_mm(xq, gathered.operand(w), x.dtype)[:M].reshape(*x.shape[:-1], size * w.shape[0])
+        return tuple(backend.fp4_mm(xq, gathered.operand(w), x.dtype).reshape(*x.shape[:-1], size * w.shape[0])
                      for w in weights)
 
     @staticmethod

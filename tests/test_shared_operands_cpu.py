@@ -29,6 +29,8 @@ def counted(monkeypatch):
 LAYERS = {
     "linear": lambda x, w, recipe: backend.nvfp4_linear(x, w, None, recipe),
     "shared input": lambda x, w, recipe: parallel.SharedInputFp4Linears.apply(x, recipe, w)[0],
+    "token parallel": lambda x, w, recipe: parallel.TokenParallelFp4Linear.apply(
+        x, SimpleNamespace(group=None, operand=lambda w: w), recipe, w)[0],
 }
 
 
