@@ -395,8 +395,9 @@ def quantize_nvfp4(x: torch.Tensor, global_scale: torch.Tensor, seed: int = -1, 
 def amax_quantize_nvfp4(x: torch.Tensor, seed: int = -1, step: int = 0, blocked: bool = False):
     """``amax_global`` and ``quantize_nvfp4`` against the scale it finds, enqueued by one library call: returns
     (packed, scales, amax [4]); the per-tensor scale is ``amax[1:2]``."""
-    packed, scales, am = _C.native("bl_nvfp4_amax_quantize", _host.amax_quantize, x, seed, step, blocked,
-                                   extra_kernels=-1 if x.numel() <= 1 << 18 else 0)      # small inputs: one kernel
+    packed, scales, am = _C.native("bl_nvfp4_amax_quantize", _host.amax_quantize, x, seed, step, blocked)
+    if x.numel() <= _host.AMAX_QUANTIZE_SMALL:           # small inputs: one kernel
+        _C.Counters.launches -= 1
     return packed, scales if blocked else scales.view(torch.float8_e4m3fn), am
 
 

@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(kQThreads, MODE == kModeSr ? 4 : 3)
 // SMs' worth of work still below four launches'.
 constexpr int kSmallCtas = 8, kSmallThreads = 512, kSmallPer = 4;
 constexpr int64_t kSmallBlocks = static_cast<int64_t>(kSmallCtas) * kSmallThreads * kSmallPer;
+static_assert(kSmallBlocks * 16 == BL_AMAX_QUANTIZE_SMALL, "the limit that the header states");
 
 template <typename T, int MODE>
 __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads, 1)

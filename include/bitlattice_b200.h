@@ -192,7 +192,9 @@ BL_API int bl_nvfp4_quantize(const void* x, int dtype, int64_t rows, int64_t col
                       uint32_t step, uint8_t* codes, uint8_t* scales, int sf_layout, int device, bl_stream_t stream);
 
 /* bl_nvfp4_amax followed by bl_nvfp4_quantize against the scale it finds (amax4[1]), enqueued by one call: the pair of
- * operators of bitlattice/backend.py:237-244 (quantize_fp4). amax4: 4 floats as bl_nvfp4_amax's out. */
+ * operators of bitlattice/backend.py:237-244 (quantize_fp4). amax4: 4 floats as bl_nvfp4_amax's out. One kernel instead
+ * of two up to BL_AMAX_QUANTIZE_SMALL values. */
+#define BL_AMAX_QUANTIZE_SMALL 262144
 BL_API int bl_nvfp4_amax_quantize(const void* x, int dtype, int64_t rows, int64_t cols, float* amax4, int64_t seed,
                            uint32_t step, uint8_t* codes, uint8_t* scales, int sf_layout, int device,
                            bl_stream_t stream);

@@ -222,3 +222,16 @@ def test_an_index_offset_of_the_counter_hash_is_a_value_of_its_step():
         step = (offset * parallel._HASH_INDEX_MUL * parallel._HASH_STEP_INV) & 0xFFFFFFFF
         for seed in (0, 77, 0x7FFFFFFF):
             assert np.array_equal(G.hash_u(idx + np.uint64(offset), seed, 0), G.hash_u(idx, seed, step))
+
+
+def test_what_is_not_a_cuda_tensor_is_refused_by_name():
+    """The calls that go through the extension module name the argument, whatever stands in its place."""
+    t = torch.zeros(16, 16)
+    for bad in (None, 1.5, np.zeros((16, 16), np.float32), t):
+        for call, name in ((lambda: _ops.amax_global(bad), "x"), (lambda: _ops.amax_quantize_nvfp4(bad), "x"),
+                           (lambda: _ops.quantize_nvfp4_4over6(bad, t), "x"), (lambda: _ops.quantize_nvfp4_t(bad, None), "x"),
+                           (lambda: _ops.requantize_nvfp4_t(bad, t, t), "packed"), (lambda: _ops.to_blocked(bad), "scales"),
+                           (lambda: _ops.dequantize(bad, t, t, None, "nvfp4", 16, 16), "packed"),
+                           (lambda: _ops.nvfp4_gemm(bad, t, t, t, t, t), "a_packed")):
+            with pytest.raises(RuntimeError, match=f"^{name} must be a CUDA tensor"):
+                call()

@@ -269,3 +269,22 @@ def test_amax_finds_every_position(n, dtype):
     assert _ops.amax_global(x)[0].item() == (0.5 if n > 1 else 0.0)
     x[n // 3] = float("inf")
     assert _ops.amax_global(x)[0].item() == float("inf")
+
+
+def test_host_calls_keep_their_integers_and_errors():
+    """Seeds and steps of any integer-like type, taken modulo 2^64; refusals as Python exceptions of the usual types."""
+    x = torch.randn(16, 64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).to(torch.bfloat16)
+    want = _ops.amax_quantize_nvfp4(x, 7, 3)
+    for seed, step in ((np.int64(7), np.int32(3)), (7.0, 3.0), (torch.tensor(7), True + 2), (7 + (1 << 64), 3 + (5 << 32)), (7, 3 - (1 << 32))):
+        for a, b in zip(_ops.amax_quantize_nvfp4(x, seed, step), want):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    for pad_rows in (0, -32):
+        with pytest.raises(RuntimeError, match="pad_rows"):
+            _ops.quantize_nvfp4_t(x, None, pad_rows=pad_rows)
+    packed, scales, am = want
+    torch.cuda.set_per_process_memory_fraction(0.5)          # (the allocator refuses before it asks the device)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            _ops.dequantize(packed, scales, am[1:2], None, "nvfp4", 1 << 22, 1 << 22)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
