@@ -451,8 +451,13 @@ __device__ __forceinline__ void sr_pair(f32x2 x, uint32_t ha, uint32_t hb, float
 
 constexpr uint32_t kSrUndecided = 0x20000u;
 
+// Whether an element of a block times inv can be a NaN (a NaN among them, infinity times 0, 0 times infinity), whose bit
+// pattern sr_pair's sum would carry into a zero: e2m1_sr8_exact gives it the largest level, whatever its neighbours draw.
+// m: the block's maximum with NaN kept (max_abs16_nan).
+__device__ __forceinline__ bool sr_special(float m, float inv) { return !(m * inv < __int_as_float(0x7F800000)); }
+
 // one block, elements (2 j, 2 j + 1) in the pairs
-__device__ __forceinline__ uint2 e2m1_sr16(const float v[16], float inv, uint32_t key, uint32_t idx0) {
+__device__ __forceinline__ uint2 e2m1_sr16(const float v[16], float inv, uint32_t key, uint32_t idx0, bool special) {
   const uint32_t h0 = idx0 * 0x27D4EB2Fu + key;
   const f32x2 inv2 = pk(inv, inv);
   uint32_t w[2];
@@ -461,7 +466,7 @@ __device__ __forceinline__ uint2 e2m1_sr16(const float v[16], float inv, uint32_
     const float* p = v + 8 * half;
     const uint32_t h = h0 + static_cast<uint32_t>(8 * half) * 0x27D4EB2Fu;
     float l[8];
-    uint32_t z = 0xFFFFFFFFu;
+    uint32_t z = special ? 0u : 0xFFFFFFFFu;
 #pragma unroll
     for (int i = 0; i < 8; i += 2)
       sr_pair(mul2p(pk(p[i], p[i + 1]), inv2), h + static_cast<uint32_t>(i) * 0x27D4EB2Fu,
@@ -475,7 +480,7 @@ __device__ __forceinline__ uint2 e2m1_sr16(const float v[16], float inv, uint32_
 }
 
 // two blocks at once, one in each lane of the pairs; h0a, h0b: first hash words of their first elements
-__device__ __forceinline__ void e2m1_sr16x2(const f32x2 v[16], float inv_a, float inv_b, uint32_t h0a, uint32_t h0b,
+__device__ __forceinline__ void e2m1_sr16x2(const f32x2 v[16], float inv_a, float inv_b, uint32_t h0a, uint32_t h0b, bool special,
                                             uint32_t ca[2], uint32_t cb[2]) {
   const f32x2 inv2 = pk(inv_a, inv_b);
 #pragma unroll
@@ -483,7 +488,7 @@ __device__ __forceinline__ void e2m1_sr16x2(const f32x2 v[16], float inv_a, floa
     const f32x2* p = v + 8 * half;
     const uint32_t ha = h0a + static_cast<uint32_t>(8 * half) * 0x27D4EB2Fu, hb = h0b + static_cast<uint32_t>(8 * half) * 0x27D4EB2Fu;
     float la[8], lb[8];
-    uint32_t z = 0xFFFFFFFFu;
+    uint32_t z = special ? 0u : 0xFFFFFFFFu;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       sr_pair(mul2p(p[i], inv2), ha + static_cast<uint32_t>(i) * 0x27D4EB2Fu, hb + static_cast<uint32_t>(i) * 0x27D4EB2Fu,
@@ -500,7 +505,7 @@ __device__ __forceinline__ void e2m1_sr16x2(const f32x2 v[16], float inv_a, floa
   }
 }
 
-// max |v[i]| of 16 values (three-input maximum of this architecture)
+// max |v[i]| of 16 values (three-input maximum of this architecture): a NaN is ignored, unless all are (0)
 __device__ __forceinline__ float max_abs3(float a, float b, float c) {
   float r;
   asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -510,6 +515,17 @@ __device__ __forceinline__ float max_abs16(const float v[16]) {
   const float a = max_abs3(v[0], v[1], v[2]), b = max_abs3(v[3], v[4], v[5]), c = max_abs3(v[6], v[7], v[8]),
               d = max_abs3(v[9], v[10], v[11]), e = max_abs3(v[12], v[13], v[14]);
   return max_abs3(max_abs3(a, b, c), max_abs3(d, e, v[15]), 0.0f);
+}
+// the same with NaN kept
+__device__ __forceinline__ float max_abs3_nan(float a, float b, float c) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max_abs16_nan(const float v[16]) {
+  const float a = max_abs3_nan(v[0], v[1], v[2]), b = max_abs3_nan(v[3], v[4], v[5]), c = max_abs3_nan(v[6], v[7], v[8]),
+              d = max_abs3_nan(v[9], v[10], v[11]), e = max_abs3_nan(v[12], v[13], v[14]);
+  return max_abs3_nan(max_abs3_nan(a, b, c), max_abs3_nan(d, e, v[15]), 0.0f);
 }
 
 // ---------------------------------------------------------------------------------------------- device: dense loads

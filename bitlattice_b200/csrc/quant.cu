@@ -167,7 +167,7 @@ __device__ __forceinline__ float fos_candidate(const float v[16], float se, uint
 
 // One block of 16 values v[i] * pre (pre: 1 or a power of two) -> 16 codes and the scale byte.
 // kModeRtn: reference.quantize 'rtn'. kModeSr: fp4ref.quantize 'sr' (idx0 = flat index of v[0]). kModeFosMse /
-// kModeFosMae: fp4ref.quantize 'rtn' with four_over_six (pre must be 1).
+// kModeFosMae: fp4ref.quantize 'rtn' with four_over_six (pre must be 1). amax: max |v|, with kModeSr or NaN if there is one.
 template <int MODE>
 __device__ __forceinline__ uint2 quantize_block(const float v[16], float amax, float pre, float g, float rg, uint32_t key,
                                                 uint32_t idx0, uint32_t* scale) {
@@ -178,11 +178,12 @@ __device__ __forceinline__ uint2 quantize_block(const float v[16], float amax, f
     *scale = sb;
     return e2m1_rtn16(v, pre, se, rcp_approx(se));
   } else if constexpr (MODE == kModeSr) {
-    const uint32_t sb = e4m3_encode(div_rn(div_rn(amax, 6.0f, kInv6), g, rg));
+    const float finite = __builtin_expect(amax != amax, 0) ? max_abs16(v) * pre : amax;      // the scale ignores NaN
+    const uint32_t sb = e4m3_encode(div_rn(div_rn(finite, 6.0f, kInv6), g, rg));
     const float t = e4m3_decode(sb) * g;
     const float inv = t > 0.0f ? __frcp_rn(t) : 0.0f;
     *scale = sb;
-    return e2m1_sr16(v, inv * pre, key, idx0);
+    return e2m1_sr16(v, inv * pre, key, idx0, sr_special(amax, inv));
   } else {
     const uint32_t b6 = e4m3_encode(div_rn(div_rn(amax, 6.0f, kInv6), g, rg));
     const uint32_t b4 = e4m3_encode(div_rn(amax * 0.25f, g, rg));
@@ -207,17 +208,20 @@ __device__ __forceinline__ void load_raw16(const T* p, Raw16<T>& r) {
   for (int i = 0; i < static_cast<int>(sizeof(T)); ++i) r.q[i] = __ldcs(reinterpret_cast<const uint4*>(p) + i);
 }
 
-// max |element|: the 16-bit types two at a time, without unpacking
-template <typename T>
+// max |element|, KEEP_NAN: or NaN; the 16-bit types two at a time, without unpacking
+template <typename T, bool KEEP_NAN>
 __device__ __forceinline__ float max_abs_raw16(const Raw16<T>& r, const float v[16]) {
-  if constexpr (sizeof(T) == 4) return max_abs16(v);
+  if constexpr (sizeof(T) == 4) return KEEP_NAN ? max_abs16_nan(v) : max_abs16(v);
   else {
     const uint32_t* w = reinterpret_cast<const uint32_t*>(r.q);
     using T2 = typename std::conditional<std::is_same<T, __nv_bfloat16>::value, __nv_bfloat162, __half2>::type;
     T2 m = __habs2(*reinterpret_cast<const T2*>(&w[0]));
 #pragma unroll
-    for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const T2*>(&w[i])));
-    return fmaxf(to_f<T>(m.x), to_f<T>(m.y));
+    for (int i = 1; i < 8; ++i) {
+      const T2 e = __habs2(*reinterpret_cast<const T2*>(&w[i]));
+      m = KEEP_NAN ? __hmax2_nan(m, e) : __hmax2(m, e);
+    }
+    return KEEP_NAN ? max_abs3_nan(to_f<T>(m.x), to_f<T>(m.y), 0.0f) : fmaxf(to_f<T>(m.x), to_f<T>(m.y));
   }
 }
 
@@ -270,7 +274,7 @@ __global__ void __launch_bounds__(kQThreads, MODE == kModeSr ? 4 : 3)
     float v[16];
     unpack_raw16(cur, v);
     uint32_t sb;
-    const uint2 out = quantize_block<MODE>(v, max_abs_raw16<T>(cur, v), 1.0f, g, rg, key, static_cast<uint32_t>(r * cols + cb * 16), &sb);
+    const uint2 out = quantize_block<MODE>(v, max_abs_raw16<T, MODE == kModeSr>(cur, v), 1.0f, g, rg, key, static_cast<uint32_t>(r * cols + cb * 16), &sb);
     __stcs(reinterpret_cast<uint2*>(codes + r * (cols / 2)) + cb, out);
     const int64_t sf_row = layout == BL_SF_ROWMAJOR ? r * cols16
                                                     : (r >> 7) * nc * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4;
@@ -311,9 +315,9 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
     if (b < blocks) {
       float v[16];
       unpack_raw16(raw[k], v);
-      bmax[k] = max_abs_raw16<T>(raw[k], v);
+      bmax[k] = max_abs_raw16<T, MODE == kModeSr>(raw[k], v);
+      m = fmaxf(m, MODE == kModeSr && bmax[k] != bmax[k] ? max_abs16(v) : bmax[k]);
     }
-    m = fmaxf(m, bmax[k]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -618,6 +622,14 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
       float va[16], vb[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) upk(v2[i], va[i], vb[i]);
+      amax_a = SR ? max_abs16_nan(va) : max_abs16(va);
+      amax_b = SR ? max_abs16_nan(vb) : max_abs16(vb);
+    }
+    const float nan_a = amax_a, nan_b = amax_b;
+    if (SR && __builtin_expect(nan_a != nan_a || nan_b != nan_b, 0)) {         // the scales ignore NaN
+      float va[16], vb[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) upk(v2[i], va[i], vb[i]);
       amax_a = max_abs16(va);
       amax_b = max_abs16(vb);
     }
@@ -627,10 +639,11 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
     const uint32_t sb = e4m3_encode(div_rn(SR ? fb : fmaxf(fb, 1e-12f), g, rg));
     const float ta = e4m3_decode(sa) * g, tb = e4m3_decode(sb) * g;
     uint32_t ca[2], cb[2];
-    if constexpr (SR)
-      e2m1_sr16x2(v2, ta > 0.0f ? __frcp_rn(ta) : 0.0f, tb > 0.0f ? __frcp_rn(tb) : 0.0f, idx_a * 0x27D4EB2Fu + key,
-                  idx_b * 0x27D4EB2Fu + key, ca, cb);
-    else
+    if constexpr (SR) {
+      const float inv_a = ta > 0.0f ? __frcp_rn(ta) : 0.0f, inv_b = tb > 0.0f ? __frcp_rn(tb) : 0.0f;
+      e2m1_sr16x2(v2, inv_a, inv_b, idx_a * 0x27D4EB2Fu + key, idx_b * 0x27D4EB2Fu + key,
+                  sr_special(nan_a, inv_a) || sr_special(nan_b, inv_b), ca, cb);
+    } else
       e2m1_rtn16x2(v2, ta, tb, rcp_approx(ta), rcp_approx(tb), ca, cb);
     s_codes[2 * kp][mb] = make_uint2(ca[0], ca[1]);
     s_codes[2 * kp + 1][mb] = make_uint2(cb[0], cb[1]);

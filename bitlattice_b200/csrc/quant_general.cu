@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kGenThreads) general_kernel(GenArgs A) {
       if (A.mode == BL_Q_SR) {
         const uint32_t idx0 = static_cast<uint32_t>(static_cast<uint64_t>(r) * static_cast<uint64_t>(A.cols) +
                                                     static_cast<uint64_t>(col0 + 16 * blk));
-        codes = e2m1_sr16(v, inv, A.key, idx0);
+        codes = e2m1_sr16(v, inv, A.key, idx0, sr_special(max_abs16_nan(v), inv));
       } else if (A.mode == BL_Q_EDEN) {
         float xx, xr;
         eden_sums(v, codes, t, xx, xr);
@@ -529,8 +529,10 @@ __global__ void __launch_bounds__(kGenThreads, 3) rotated_kernel(GenArgs A) {
       if (A.mode == BL_Q_SR) {
         const uint32_t idx = static_cast<uint32_t>(static_cast<uint64_t>(row0) * static_cast<uint64_t>(A.cols) +
                                                    static_cast<uint64_t>(col0 + 16 * b));
-        codes[0] = e2m1_sr16(va, inv[0], A.key, idx + static_cast<uint32_t>(pair[0]) * static_cast<uint32_t>(A.cols));
-        codes[1] = e2m1_sr16(vb, inv[1], A.key, idx + static_cast<uint32_t>(pair[1]) * static_cast<uint32_t>(A.cols));
+        codes[0] = e2m1_sr16(va, inv[0], A.key, idx + static_cast<uint32_t>(pair[0]) * static_cast<uint32_t>(A.cols),
+                             sr_special(max_abs16_nan(va), inv[0]));
+        codes[1] = e2m1_sr16(vb, inv[1], A.key, idx + static_cast<uint32_t>(pair[1]) * static_cast<uint32_t>(A.cols),
+                             sr_special(max_abs16_nan(vb), inv[1]));
       } else if (A.mode == BL_Q_EDEN) {
         float2 xx, xr;
         eden_sums2(v, codes, t, xx, xr);

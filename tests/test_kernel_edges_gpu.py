@@ -288,3 +288,62 @@ def test_host_calls_keep_their_integers_and_errors():
             _ops.dequantize(packed, scales, am[1:2], None, "nvfp4", 1 << 22, 1 << 22)
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def _special_values(shape, dtype, rng):
+    """Normal values, 1 % NaN of either sign and 1 % infinities, and blocks of 16 of nothing but NaN along either side."""
+    v = rng.standard_normal(shape).astype(np.float32)
+    at = rng.random(shape)
+    v[at < 0.01] = np.nan
+    v[at < 0.005] = -np.nan
+    v[at > 0.99] = np.inf
+    v[at > 0.995] = -np.inf
+    v[3, 32:48] = np.nan
+    v[64:80, 5] = np.nan
+    return torch.from_numpy(v).to(dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_stochastic_rounding_of_nan_and_infinity(dtype):
+    """A NaN takes the largest level and is ignored by every maximum, whatever its neighbours draw; an infinity is the
+    largest level of its sign, or a NaN where the scale of its block is infinite as well. Rows, transposed with an even and
+    an odd number of columns and rotated, and the one-launch form for small inputs."""
+    rng = np.random.default_rng(19)
+    x = _special_values((512, 512), dtype, rng)
+    xf = x.float().numpy()
+    for g in (0.0011, 0.11):
+        rc, rs, _ = oracle.quantize_rows(xf, g, "sr", seed=11)
+        packed, sc = _ops.quantize_nvfp4(x.cuda(), dev(np.array([g], np.float32)), seed=11)
+        assert np.array_equal(host(packed), rc) and np.array_equal(host(sc), rs)
+    H = oracle.hadamard16()
+    for cols, h in ((512, None), (511, None), (512, H)):
+        part = x[:, :cols].contiguous()
+        rc, rs = oracle.quantize_t(part.float().numpy(), h, oracle.global_from_bound(0.02), "sr", seed=5)
+        packed, sc, _ = _ops.quantize_nvfp4_t(part.cuda(), dev(h.astype(np.float32)) if h is not None else None, 5, 0,
+                                              dev(np.array([0.02], np.float32)))
+        assert np.array_equal(host(packed), rc) and np.array_equal(host(sc), rs)
+    for part in (x[:40], x[:40].nan_to_num(posinf=1.0, neginf=-1.0, nan=float("nan"))):
+        rc, rs, rg = oracle.quantize_rows(part.float().numpy(), None, "sr", seed=3)
+        packed, sc, am = _ops.amax_quantize_nvfp4(part.cuda(), 3)
+        assert am[1].item() == rg and np.array_equal(host(packed), rc) and np.array_equal(host(sc), rs)
+
+
+@pytest.mark.parametrize("rotate", [False, True])
+@pytest.mark.parametrize("transpose", [False, True])
+def test_general_stochastic_rounding_of_nan(rotate, transpose):
+    """The general quantizer: NaN takes the largest level, and what shares no block (rotated: no segment of 128) with one
+    keeps its code."""
+    x = torch.randn(256, 256, generator=torch.Generator().manual_seed(2)).cuda()
+    bad = x.clone()
+    bad[7, 20] = bad[200, 131] = float("nan")
+    given = torch.tensor([0.002], device="cuda")
+    kw = dict(transpose=transpose, mode="sr", rotate=rotate, seed=4, rotate_seed=9 if rotate else -1, given=given)
+    clean, dirty = (host(_ops.nvfp4_quantize_general(v, **kw)[0]) for v in (x, bad))
+    clean, dirty = (np.stack([c & 15, c >> 4], -1).reshape(256, 256) for c in (clean, dirty))
+    span = 128 if rotate else 16
+    for r, c in ((20, 7), (131, 200)) if transpose else ((7, 20), (200, 131)):
+        hit = dirty[r, c // span * span:][:span] if rotate else dirty[r, c:c + 1]
+        assert (hit == 7).all()
+        lo = c // span * span
+        dirty[r, lo:lo + span] = clean[r, lo:lo + span]
+    assert np.array_equal(clean, dirty)
