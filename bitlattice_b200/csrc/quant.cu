@@ -789,7 +789,8 @@ __global__ void __launch_bounds__(kQThreads) requantize_t_kernel(const uint8_t* 
   const int64_t kr = k0 + row, nn = n0 + 16 * b0, cols16 = N / 16;
   if (kr >= K || nn >= N) return;
   uint2* dst = reinterpret_cast<uint2*>(codes + kr * (N / 2) + nn / 2);
-  if (nn + 64 <= N && (cols16 & 3) == 0) {                   // rows of whole 32-byte pieces: the usual case
+  // rows of whole 32-byte pieces, scales at a whole word: the usual case
+  if (nn + 64 <= N && (cols16 & 3) == 0 && (reinterpret_cast<uintptr_t>(scales) & 3u) == 0) {
     const uint2 c0 = s_codes[b0][row], c1 = s_codes[b0 + 1][row], c2 = s_codes[b0 + 2][row], c3 = s_codes[b0 + 3][row];
     reinterpret_cast<uint4*>(dst)[0] = make_uint4(c0.x, c0.y, c1.x, c1.y);
     reinterpret_cast<uint4*>(dst)[1] = make_uint4(c2.x, c2.y, c3.x, c3.y);

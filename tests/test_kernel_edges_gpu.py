@@ -37,6 +37,25 @@ def test_requantize_t_ties_and_edges(N, K, g):
         assert gout.item() == np.float32(g)
 
 
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_requantize_t_scales_at_any_address(shift, layout):
+    """Scale buffers that start inside a word are written by bytes, and nothing beside them is."""
+    N, K, g = 128, 64, 0.0137
+    rng = np.random.default_rng(5)
+    codes, scales = rng.integers(0, 256, (N, K // 2), dtype=np.uint8), rng.integers(0x28, 0x50, (N, K // 16), dtype=np.uint8)
+    rc, rs = oracle.requantize_t(codes, scales, g)
+    want = (oracle.to_blocked(rs) if layout else rs).reshape(-1)
+    gd, out, gout = dev(np.array([g], np.float32)), torch.empty(K, N // 2, dtype=torch.uint8, device="cuda"), torch.empty(1, device="cuda")
+    raw = torch.full((want.size + 16,), 0xEE, dtype=torch.uint8, device="cuda")
+    packed, sc = dev(codes), dev(scales)
+    _C.call("bl_nvfp4_requantize_t", packed.data_ptr(), sc.data_ptr(), gd.data_ptr(), N, K, out.data_ptr(), raw.data_ptr() + 8 + shift,
+            gout.data_ptr(), layout, 0, torch.cuda.current_stream().cuda_stream)
+    got = host(raw)
+    assert np.array_equal(host(out), rc) and np.array_equal(got[8 + shift:8 + shift + want.size], want)
+    assert (got[:8 + shift] == 0xEE).all() and (got[8 + shift + want.size:] == 0xEE).all()
+
+
 @pytest.mark.parametrize("rows,cols16", [(1, 1), (5, 4), (128, 4), (129, 8), (300, 12), (127, 6), (257, 64)])
 def test_to_blocked_words_and_bytes(rows, cols16):
     s = np.random.default_rng(rows).integers(0, 256, (rows, cols16), dtype=np.uint8)
