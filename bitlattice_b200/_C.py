@@ -86,6 +86,7 @@ _SIGNATURES = {
     "bl_swiglu_bwd": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int64,
                                   _c.c_int, _c.c_void_p]),
     "bl_selftest_division": (_c.c_int, [_c.c_uint64, _c.c_uint32, _c.POINTER(_c.c_uint64), _c.c_int]),
+    "bl_selftest_division_slice": (_c.c_int, [_c.c_uint32, _c.POINTER(_c.c_uint64), _c.c_int]),
 }
 
 _lib = None

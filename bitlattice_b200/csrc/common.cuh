@@ -162,9 +162,11 @@ __device__ __forceinline__ uint32_t e2m1_code_sr(float v, float u) {
 // Research and Development 34, 1990; the case of a divisor known in advance: Brisebarre, Muller and Raina, "Accelerating
 // correctly rounded floating-point division when the divisor is known in advance", IEEE Transactions on Computers 53,
 // 2004): the product q = RN(x ry) is off by less than two units in the last place, its residual r = x - y q is formed by
-// one fused multiply-add, and RN(q + r ry) is the correctly rounded quotient. Run over all 2^46 pairs of fp32
-// significands on a B200 it agreed with the plain division on every one; exponents only scale the three operations while
-// nothing leaves the normal range, which the callers (or the check below) establish.
+// one fused multiply-add, and RN(q + r ry) is the correctly rounded quotient. The theorems leave the divisors open for which
+// q is not a neighbour of the quotient, so every pair of fp32 significands is compared with the plain division
+// (bl_selftest_division_slice; 2^46 pairs, none differs on a B200). Exponents only scale the three operations while
+// nothing leaves the normal range and the residual, a multiple of 2^-48 x or less, is a float: |x| > 2^-100, a normal ry, a
+// quotient far from either end. The callers of div2p establish that; div_rn checks it.
 static __device__ __noinline__ float div_general(float x, float y) { return x / y; }
 
 __device__ __forceinline__ float div_rn(float x, float y, float ry) {
@@ -172,7 +174,8 @@ __device__ __forceinline__ float div_rn(float x, float y, float ry) {
   const float q = fmaf(fmaf(-y, q0, x), ry, q0);
   const float aq = fabsf(q0);
   // zero, tiny, huge or non-finite: the general path, kept out of line so that it costs nothing when not taken
-  if (__builtin_expect(!(aq > 1e-30f && aq < 1e30f), 0)) return div_general(x, y);
+  const bool in_range = aq > 1e-30f && aq < 1e30f && fabsf(x) > 7.8886091e-31f && fabsf(ry) >= 1.1754943508222875e-38f;
+  if (__builtin_expect(!in_range, 0)) return div_general(x, y);
   return q;
 }
 

@@ -898,7 +898,8 @@ __global__ void to_blocked_kernel(const uint8_t* __restrict__ scales, int64_t ro
   }
 }
 
-// self-test of div_rn against the plain division on pseudo-random operands (magnitudes 2^-40 .. 2^40, both signs)
+// self-test of div_rn against the plain division on pseudo-random operands: magnitudes 2^-40 .. 2^40, both signs, and any bit
+// patterns (subnormal numbers, zeros, infinities)
 __global__ void selftest_division_kernel(uint64_t n, uint32_t seed, unsigned long long* mismatches) {
   unsigned long long bad = 0;
   for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
@@ -912,6 +913,8 @@ __global__ void selftest_division_kernel(uint64_t n, uint32_t seed, unsigned lon
     const float y = __uint_as_float((b & 0x807FFFFFu) | (eb << 23));
     const float q = div_rn(x, y, __frcp_rn(y));
     bad += __float_as_uint(q) != __float_as_uint(x / y);
+    const float xw = __uint_as_float(a), yw = __uint_as_float(b), qw = xw / yw;
+    bad += qw == qw && __float_as_uint(div_rn(xw, yw, __frcp_rn(yw))) != __float_as_uint(qw);
     // the packed sequence (no range check of its own): both lanes, inside the range its callers establish
     const float x2 = __uint_as_float(__float_as_uint(x) ^ 0x00155555u);
     float q0, q1;
@@ -944,6 +947,20 @@ __global__ void selftest_division_kernel(uint64_t n, uint32_t seed, unsigned lon
     upk(add2p(pk(x2, x), prod2p(pk(x, x2), pk(x, x2))), e0, e1);
     bad += __float_as_uint(e0) != __float_as_uint(__fadd_rn(x2, __fmul_rn(x, x)));
     bad += __float_as_uint(e1) != __float_as_uint(__fadd_rn(x, __fmul_rn(x2, x2)));
+  }
+  if (bad) atomicAdd(mismatches, bad);
+}
+
+// div2p on every fp32 significand as dividend and 2^17 of them (those of the slice) as divisors, exponents 0
+__global__ void __launch_bounds__(256) selftest_division_slice_kernel(uint32_t slice, unsigned long long* mismatches) {
+  const float y = __uint_as_float(0x3F800000u | (slice << 17) | (blockIdx.x * 256u + threadIdx.x));
+  const f32x2 ny = pk(-y, -y), ry = pk(__frcp_rn(y), __frcp_rn(y));
+  unsigned long long bad = 0;
+  for (uint32_t i = 0; i < (1u << 22); ++i) {
+    const float x0 = __uint_as_float(0x3F800000u | i), x1 = __uint_as_float(0x3FC00000u | i);
+    float q0, q1;
+    upk(div2p(pk(x0, x1), ny, ry), q0, q1);
+    bad += (q0 != x0 / y) + (q1 != x1 / y);
   }
   if (bad) atomicAdd(mismatches, bad);
 }
@@ -1205,14 +1222,13 @@ extern "C" int bl_nvfp4_scales_to_blocked(const uint8_t* scales, int64_t rows, i
   return 0;
 }
 
-extern "C" int bl_selftest_division(uint64_t n, uint32_t seed, uint64_t* mismatches, int device) {
-  BL_REQUIRE(mismatches != nullptr && n > 0, "selftest_division: null output or empty range");
-  BL_DEVICE(device);
+template <typename Launch>
+static int selftest(uint64_t* mismatches, Launch&& launch) {
   unsigned long long* d = nullptr;
   BL_CUDA(cudaMalloc(&d, sizeof(unsigned long long)));
   cudaError_t rc = cudaMemset(d, 0, sizeof(unsigned long long));
   if (rc == cudaSuccess) {
-    selftest_division_kernel<<<sm_count(device) * 8, 256>>>(n, seed, d);
+    launch(d);
     rc = cudaGetLastError();
   }
   unsigned long long h = 0;
@@ -1221,4 +1237,16 @@ extern "C" int bl_selftest_division(uint64_t n, uint32_t seed, uint64_t* mismatc
   BL_CUDA(rc);
   *mismatches = h;
   return 0;
+}
+
+extern "C" int bl_selftest_division(uint64_t n, uint32_t seed, uint64_t* mismatches, int device) {
+  BL_REQUIRE(mismatches != nullptr && n > 0, "selftest_division: null output or empty range");
+  BL_DEVICE(device);
+  return selftest(mismatches, [&](unsigned long long* d) { selftest_division_kernel<<<sm_count(device) * 8, 256>>>(n, seed, d); });
+}
+
+extern "C" int bl_selftest_division_slice(uint32_t slice, uint64_t* mismatches, int device) {
+  BL_REQUIRE(mismatches != nullptr && slice < 64, "selftest_division_slice: null output or no such slice (%u of 64)", slice);
+  BL_DEVICE(device);
+  return selftest(mismatches, [&](unsigned long long* d) { selftest_division_slice_kernel<<<512, 256>>>(slice, d); });
 }

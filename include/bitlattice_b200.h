@@ -8,7 +8,7 @@
  *     buffer, outputs included) -- scratch memory, where an operation needs some, is passed in and its size comes
  *     from the matching *_scratch_bytes function. Two exceptions, both stated at their declarations:
  *     bl_nvfp4_lattice_update_fixed_scratch keeps its scratch in an array inside the library image, and the
- *     diagnostic bl_selftest_division makes a temporary 8-byte allocation;
+ *     diagnostics bl_selftest_division* make a temporary 8-byte allocation;
  *   - all buffers are contiguous and 16-byte aligned; shapes are validated before anything is launched;
  *   - work is enqueued on `stream` of CUDA device `device` and the call returns without synchronizing;
  *   - the return value is 0 on success, non-zero on failure; bl_last_error() then describes the failure
@@ -355,6 +355,10 @@ BL_API int bl_nvfp4_gemm_select(int kernel);
  * plain division on n pseudo-random operand pairs (synchronously, with a temporary 8-byte device allocation) and
  * stores the number of results that differ in any bit; the test-suite requires 0. */
 BL_API int bl_selftest_division(uint64_t n, uint32_t seed, uint64_t* mismatches, int device);
+
+/* The same for every fp32 significand as dividend and one of 64 slices of them as divisors (2^40 pairs, about a second):
+ * all slices together are all pairs. */
+BL_API int bl_selftest_division_slice(uint32_t slice, uint64_t* mismatches, int device);
 
 #ifdef __cplusplus
 }

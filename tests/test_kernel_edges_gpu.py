@@ -366,3 +366,13 @@ def test_general_stochastic_rounding_of_nan(rotate, transpose):
         lo = c // span * span
         dirty[r, lo:lo + span] = clean[r, lo:lo + span]
     assert np.array_equal(clean, dirty)
+
+
+@pytest.mark.parametrize("slice_", [0, 21, 42, 63])
+def test_division_on_every_significand(slice_):
+    """The packed division on all dividends by 2^17 divisors; the 64 slices together are all 2^46 pairs of significands (run
+    in full when the routine changes: a minute on a B200)."""
+    import ctypes
+    bad = ctypes.c_uint64(1)
+    _C.call("bl_selftest_division_slice", slice_, ctypes.byref(bad), 0)
+    assert bad.value == 0
