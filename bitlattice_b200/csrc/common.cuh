@@ -179,6 +179,36 @@ __device__ __forceinline__ float div_rn(float x, float y, float ry) {
   return q;
 }
 
+// The two divisions of a block scale, amax / 6 and the quotient by the per-tensor scale g, checked by their quotients alone:
+// the first's bounds its dividend (6e-30 > 2^-100), and rg = scale_rcp(g) is a NaN, which fails every check, unless g is
+// large enough (1e-12, the least that is ever computed) for the second's to do so. With the dividends checked themselves the
+// row quantizers took 1 to 2 % longer.
+constexpr float kInv6 = 0.16666667163372039794921875f;   // the float nearest to 1/6
+constexpr float kScaleQuotient = 8.6736174e-19f;         // 2^-60: 2^-60 * 1e-12 > 2^-100; a block 2^69 below the maximum
+
+__device__ __forceinline__ float scale_rcp(float g) {
+  return g >= 1e-12f && g < 8.507059e37f ? __frcp_rn(g) : __int_as_float(0x7FFFFFFF);
+}
+__device__ __forceinline__ float div_checked(float x, float y, float ry, float lo, bool& ok) {
+  const float q0 = x * ry, aq = fabsf(q0);
+  ok = ok && aq > lo && aq < 1e30f;
+  return fmaf(fmaf(-y, q0, x), ry, q0);
+}
+__device__ __forceinline__ float div_six(float x) {
+  bool ok = true;
+  const float q = div_checked(x, 6.0f, kInv6, 1e-30f, ok);
+  return __builtin_expect(ok, 1) ? q : div_general(x, 6.0f);
+}
+__device__ __forceinline__ float div_scale(float x, float g, float rg) {
+  bool ok = true;
+  const float q = div_checked(x, g, rg, kScaleQuotient, ok);
+  return __builtin_expect(ok, 1) ? q : div_general(x, g);
+}
+// amax / 6 / g; ok: both quotients are exact (amax is neither zero nor tiny beside g, infinite nor a NaN)
+__device__ __forceinline__ float div_block_scale(float amax, float g, float rg, bool& ok) {
+  return div_checked(div_checked(amax, 6.0f, kInv6, 1e-30f, ok), g, rg, kScaleQuotient, ok);
+}
+
 // ---------------------------------------------------------------------------------------------- device: fp32 pairs
 // Two independent fp32 operations per instruction, each lane rounded to nearest like the scalar operation (the fused
 // multiply-add is written out only where a single rounding is wanted: the residuals of the divisions).
@@ -454,13 +484,8 @@ __device__ __forceinline__ void sr_pair(f32x2 x, uint32_t ha, uint32_t hb, float
 
 constexpr uint32_t kSrUndecided = 0x20000u;
 
-// Whether an element of a block times inv can be a NaN (a NaN among them, infinity times 0, 0 times infinity), whose bit
-// pattern sr_pair's sum would carry into a zero: e2m1_sr8_exact gives it the largest level, whatever its neighbours draw.
-// m: the block's maximum with NaN kept (max_abs16_nan).
-__device__ __forceinline__ bool sr_special(float m, float inv) { return !(m * inv < __int_as_float(0x7F800000)); }
-
-// one block, elements (2 j, 2 j + 1) in the pairs
-__device__ __forceinline__ uint2 e2m1_sr16(const float v[16], float inv, uint32_t key, uint32_t idx0, bool special) {
+// one block, elements (2 j, 2 j + 1) in the pairs; special: a product can be a NaN
+__device__ __forceinline__ uint2 e2m1_sr16(const float v[16], float inv, uint32_t key, uint32_t idx0, bool special = false) {
   const uint32_t h0 = idx0 * 0x27D4EB2Fu + key;
   const f32x2 inv2 = pk(inv, inv);
   uint32_t w[2];
@@ -483,7 +508,7 @@ __device__ __forceinline__ uint2 e2m1_sr16(const float v[16], float inv, uint32_
 }
 
 // two blocks at once, one in each lane of the pairs; h0a, h0b: first hash words of their first elements
-__device__ __forceinline__ void e2m1_sr16x2(const f32x2 v[16], float inv_a, float inv_b, uint32_t h0a, uint32_t h0b, bool special,
+__device__ __forceinline__ void e2m1_sr16x2(const f32x2 v[16], float inv_a, float inv_b, uint32_t h0a, uint32_t h0b,
                                             uint32_t ca[2], uint32_t cb[2]) {
   const f32x2 inv2 = pk(inv_a, inv_b);
 #pragma unroll
@@ -491,7 +516,7 @@ __device__ __forceinline__ void e2m1_sr16x2(const f32x2 v[16], float inv_a, floa
     const f32x2* p = v + 8 * half;
     const uint32_t ha = h0a + static_cast<uint32_t>(8 * half) * 0x27D4EB2Fu, hb = h0b + static_cast<uint32_t>(8 * half) * 0x27D4EB2Fu;
     float la[8], lb[8];
-    uint32_t z = special ? 0u : 0xFFFFFFFFu;
+    uint32_t z = 0xFFFFFFFFu;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       sr_pair(mul2p(p[i], inv2), ha + static_cast<uint32_t>(i) * 0x27D4EB2Fu, hb + static_cast<uint32_t>(i) * 0x27D4EB2Fu,
@@ -529,6 +554,39 @@ __device__ __forceinline__ float max_abs16_nan(const float v[16]) {
   const float a = max_abs3_nan(v[0], v[1], v[2]), b = max_abs3_nan(v[3], v[4], v[5]), c = max_abs3_nan(v[6], v[7], v[8]),
               d = max_abs3_nan(v[9], v[10], v[11]), e = max_abs3_nan(v[12], v[13], v[14]);
   return max_abs3_nan(max_abs3_nan(a, b, c), max_abs3_nan(d, e, v[15]), 0.0f);
+}
+
+// sr_pair must not see a NaN: the sum with the draw would carry its bit pattern into a zero. Here a block that can hold one is
+// decided on 24 bits, where it takes the largest level, as in the plain expressions: no product is a NaN if the largest
+// (NaN kept) is finite.
+__device__ __forceinline__ uint2 e2m1_sr16_any(const float v[16], float inv, uint32_t key, uint32_t idx0) {
+  return e2m1_sr16(v, inv, key, idx0, !(max_abs16_nan(v) * inv < __int_as_float(0x7F800000)));
+}
+
+// Stochastic codes and scale byte of a block for which div_block_scale is not exact: its maximum is zero, tiny, infinite or
+// (NaN kept) unknown, or the per-tensor scale is out of range. The scale ignores a NaN, which takes the largest level.
+struct SrBlock {
+  uint2 codes;
+  uint32_t scale;
+};
+static __device__ __noinline__ SrBlock sr_block_general(float4 v0, float4 v1, float4 v2, float4 v3, float g, uint32_t h0) {
+  const float v[16] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w, v3.x, v3.y, v3.z, v3.w};
+  SrBlock out;
+  out.scale = e4m3_encode(max_abs16(v) / 6.0f / g);
+  const float t = e4m3_decode(out.scale) * g;
+  const float inv = t > 0.0f ? __frcp_rn(t) : 0.0f;
+  out.codes = make_uint2(0u, 0u);
+  if (max_abs16_nan(v) * inv != 0.0f) {                         // else nothing but zeros
+    out.codes.x = e2m1_sr8_exact(make_float4(v[0] * inv, v[1] * inv, v[2] * inv, v[3] * inv),
+                                 make_float4(v[4] * inv, v[5] * inv, v[6] * inv, v[7] * inv), h0);
+    out.codes.y = e2m1_sr8_exact(make_float4(v[8] * inv, v[9] * inv, v[10] * inv, v[11] * inv),
+                                 make_float4(v[12] * inv, v[13] * inv, v[14] * inv, v[15] * inv), h0 + 8u * 0x27D4EB2Fu);
+  }
+  return out;
+}
+__device__ __forceinline__ SrBlock sr_block_general(const float v[16], float g, uint32_t h0) {
+  return sr_block_general(make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]),
+                          make_float4(v[8], v[9], v[10], v[11]), make_float4(v[12], v[13], v[14], v[15]), g, h0);
 }
 
 // ---------------------------------------------------------------------------------------------- device: dense loads

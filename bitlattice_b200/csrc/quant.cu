@@ -83,8 +83,6 @@ __global__ void __launch_bounds__(kQThreads) amax_kernel(const T* __restrict__ x
 // 8 of the 16 values of a block held by this lane (the partner lane, xor 1, holds the other 8): returns this
 // lane's 8 codes; *scale receives the E4M3 byte of the block.
 // SR == false: reference.quantize 'rtn'. SR == true: fp4ref.quantize 'sr' (idx0 = flat index of v[0]).
-constexpr float kInv6 = 0.16666667163372039794921875f;   // the float nearest to 1/6
-
 // rg = __frcp_rn(g), shared by all blocks of a kernel
 template <bool SR>
 __device__ __forceinline__ uint32_t quantize_half_block(const float v[8], float g, float rg, uint32_t key,
@@ -165,28 +163,30 @@ __device__ __forceinline__ float fos_candidate(const float v[16], float se, uint
   return err;
 }
 
-// One block of 16 values v[i] * pre (pre: 1 or a power of two) -> 16 codes and the scale byte.
-// kModeRtn: reference.quantize 'rtn'. kModeSr: fp4ref.quantize 'sr' (idx0 = flat index of v[0]). kModeFosMse /
-// kModeFosMae: fp4ref.quantize 'rtn' with four_over_six (pre must be 1). amax: max |v|, with kModeSr or NaN if there is one.
+// One block of 16 values -> 16 codes and the scale byte; rg = scale_rcp(g). kModeRtn: reference.quantize 'rtn'. kModeSr:
+// fp4ref.quantize 'sr' (idx0 = flat index of v[0]). kModeFosMse / kModeFosMae: fp4ref.quantize 'rtn' with four_over_six.
+// amax: max |v|; with kModeSr, a NaN if there is one among them.
 template <int MODE>
-__device__ __forceinline__ uint2 quantize_block(const float v[16], float amax, float pre, float g, float rg, uint32_t key,
+__device__ __forceinline__ uint2 quantize_block(const float v[16], float amax, float g, float rg, uint32_t key,
                                                 uint32_t idx0, uint32_t* scale) {
-  amax *= pre;
   if constexpr (MODE == kModeRtn) {
-    const uint32_t sb = e4m3_encode(div_rn(fmaxf(div_rn(amax, 6.0f, kInv6), 1e-12f), g, rg));
+    const uint32_t sb = e4m3_encode(div_scale(fmaxf(div_six(amax), 1e-12f), g, rg));
     const float se = e4m3_decode(sb) * g;
     *scale = sb;
-    return e2m1_rtn16(v, pre, se, rcp_approx(se));
+    return e2m1_rtn16(v, 1.0f, se, rcp_approx(se));
   } else if constexpr (MODE == kModeSr) {
-    const float finite = __builtin_expect(amax != amax, 0) ? max_abs16(v) * pre : amax;      // the scale ignores NaN
-    const uint32_t sb = e4m3_encode(div_rn(div_rn(finite, 6.0f, kInv6), g, rg));
-    const float t = e4m3_decode(sb) * g;
-    const float inv = t > 0.0f ? __frcp_rn(t) : 0.0f;
+    bool ok = true;
+    const uint32_t sb = e4m3_encode(div_block_scale(amax, g, rg, ok));
+    if (__builtin_expect(!ok, 0)) {
+      const SrBlock b = sr_block_general(v, g, idx0 * 0x27D4EB2Fu + key);
+      *scale = b.scale;
+      return b.codes;
+    }
     *scale = sb;
-    return e2m1_sr16(v, inv * pre, key, idx0, sr_special(amax, inv));
+    return e2m1_sr16(v, __frcp_rn(e4m3_decode(sb) * g), key, idx0);
   } else {
-    const uint32_t b6 = e4m3_encode(div_rn(div_rn(amax, 6.0f, kInv6), g, rg));
-    const uint32_t b4 = e4m3_encode(div_rn(amax * 0.25f, g, rg));
+    const uint32_t b6 = e4m3_encode(div_scale(div_six(amax), g, rg));
+    const uint32_t b4 = e4m3_encode(div_scale(amax * 0.25f, g, rg));
     uint2 c6, c4;
     const float e6 = fos_candidate<MODE == kModeFosMae>(v, e4m3_decode(b6) * g, c6);
     const float e4 = fos_candidate<MODE == kModeFosMae>(v, e4m3_decode(b4) * g, c4);
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kQThreads, MODE == kModeSr ? 4 : 3)
     quantize_rows16_kernel(const T* __restrict__ x, int64_t rows, int64_t cols, const float* __restrict__ global,
                            uint32_t key, uint8_t* __restrict__ codes, uint8_t* __restrict__ scales, int layout) {
   const float g = global[0];
-  const float rg = __frcp_rn(g);
+  const float rg = scale_rcp(g);
   const int64_t cb = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;   // block column
   const int64_t cols16 = cols / 16;
   if (cb >= cols16) return;
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kQThreads, MODE == kModeSr ? 4 : 3)
     float v[16];
     unpack_raw16(cur, v);
     uint32_t sb;
-    const uint2 out = quantize_block<MODE>(v, max_abs_raw16<T, MODE == kModeSr>(cur, v), 1.0f, g, rg, key, static_cast<uint32_t>(r * cols + cb * 16), &sb);
+    const uint2 out = quantize_block<MODE>(v, max_abs_raw16<T, MODE == kModeSr>(cur, v), g, rg, key, static_cast<uint32_t>(r * cols + cb * 16), &sb);
     __stcs(reinterpret_cast<uint2*>(codes + r * (cols / 2)) + cb, out);
     const int64_t sf_row = layout == BL_SF_ROWMAJOR ? r * cols16
                                                     : (r >> 7) * nc * 512 + (r & 31) * 16 + ((r >> 5) & 3) * 4;
@@ -336,7 +336,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
   float amax = s_cta[0];
 #pragma unroll
   for (int c = 1; c < kSmallCtas; ++c) amax = fmaxf(amax, s_cta[c]);
-  const float g = fmaxf(amax / 2688.0f, 1e-12f), rg = __frcp_rn(g);
+  const float g = fmaxf(amax / 2688.0f, 1e-12f), rg = scale_rcp(g);
   if (rank == 0 && tid == 0) {
     amax4[0] = amax;
     amax4[1] = g;
@@ -351,7 +351,7 @@ __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThrea
       float v[16];
       unpack_raw16(raw[k], v);
       uint32_t sb;
-      reinterpret_cast<uint2*>(codes)[b] = quantize_block<MODE>(v, bmax[k], 1.0f, g, rg, key, static_cast<uint32_t>(b) * 16u, &sb);
+      reinterpret_cast<uint2*>(codes)[b] = quantize_block<MODE>(v, bmax[k], g, rg, key, static_cast<uint32_t>(b) * 16u, &sb);
       const int r = b / cols16;
       scales[scale_index(layout, r, b - r * cols16, cols16)] = static_cast<uint8_t>(sb);
     }
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
     }
     const float g = global_t(global, given, factor);
     if (global_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) global_out[0] = g;
-    const float rg = __frcp_rn(g);
+    const float rg = scale_rcp(g);
     f32x2 v2[16];
     if (H == nullptr) {
 #pragma unroll
@@ -625,26 +625,29 @@ __global__ void __launch_bounds__(kQThreads, 4) quantize_t3_kernel(const T* __re
       amax_a = SR ? max_abs16_nan(va) : max_abs16(va);
       amax_b = SR ? max_abs16_nan(vb) : max_abs16(vb);
     }
-    const float nan_a = amax_a, nan_b = amax_b;
-    if (SR && __builtin_expect(nan_a != nan_a || nan_b != nan_b, 0)) {         // the scales ignore NaN
-      float va[16], vb[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) upk(v2[i], va[i], vb[i]);
-      amax_a = max_abs16(va);
-      amax_b = max_abs16(vb);
-    }
     const uint32_t idx_a = static_cast<uint32_t>(static_cast<uint64_t>(k) * M + m), idx_b = idx_a + static_cast<uint32_t>(M);
-    const float fa = div_rn(amax_a, 6.0f, kInv6), fb = div_rn(amax_b, 6.0f, kInv6);
-    const uint32_t sa = e4m3_encode(div_rn(SR ? fa : fmaxf(fa, 1e-12f), g, rg));
-    const uint32_t sb = e4m3_encode(div_rn(SR ? fb : fmaxf(fb, 1e-12f), g, rg));
-    const float ta = e4m3_decode(sa) * g, tb = e4m3_decode(sb) * g;
-    uint32_t ca[2], cb[2];
+    uint32_t sa, sb, ca[2], cb[2];
     if constexpr (SR) {
-      const float inv_a = ta > 0.0f ? __frcp_rn(ta) : 0.0f, inv_b = tb > 0.0f ? __frcp_rn(tb) : 0.0f;
-      e2m1_sr16x2(v2, inv_a, inv_b, idx_a * 0x27D4EB2Fu + key, idx_b * 0x27D4EB2Fu + key,
-                  sr_special(nan_a, inv_a) || sr_special(nan_b, inv_b), ca, cb);
-    } else
+      const uint32_t ha = idx_a * 0x27D4EB2Fu + key, hb = idx_b * 0x27D4EB2Fu + key;
+      bool ok = true;
+      sa = e4m3_encode(div_block_scale(amax_a, g, rg, ok));
+      sb = e4m3_encode(div_block_scale(amax_b, g, rg, ok));
+      if (__builtin_expect(ok, 1)) {
+        e2m1_sr16x2(v2, __frcp_rn(e4m3_decode(sa) * g), __frcp_rn(e4m3_decode(sb) * g), ha, hb, ca, cb);
+      } else {
+        float va[16], vb[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) upk(v2[i], va[i], vb[i]);
+        const SrBlock a = sr_block_general(va, g, ha), b = sr_block_general(vb, g, hb);
+        sa = a.scale, ca[0] = a.codes.x, ca[1] = a.codes.y;
+        sb = b.scale, cb[0] = b.codes.x, cb[1] = b.codes.y;
+      }
+    } else {
+      sa = e4m3_encode(div_scale(fmaxf(div_six(amax_a), 1e-12f), g, rg));
+      sb = e4m3_encode(div_scale(fmaxf(div_six(amax_b), 1e-12f), g, rg));
+      const float ta = e4m3_decode(sa) * g, tb = e4m3_decode(sb) * g;
       e2m1_rtn16x2(v2, ta, tb, rcp_approx(ta), rcp_approx(tb), ca, cb);
+    }
     s_codes[2 * kp][mb] = make_uint2(ca[0], ca[1]);
     s_codes[2 * kp + 1][mb] = make_uint2(cb[0], cb[1]);
     s_scales[2 * kp][mb] = static_cast<uint8_t>(sa);
@@ -735,7 +738,7 @@ __global__ void __launch_bounds__(kQThreads) requantize_t_kernel(const uint8_t* 
         am[c] = __hmax2(am[c], __habs2(pr[c][i]));
       }
     }
-    const float rg = __frcp_rn(g);
+    const float rg = scale_rcp(g);
     uint2 out[4];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
@@ -747,7 +750,7 @@ __global__ void __launch_bounds__(kQThreads) requantize_t_kernel(const uint8_t* 
       bool ok = true;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const uint32_t sb = e4m3_encode(div_rn(div_rn(amax[e], 6.0f, kInv6), g, rg));
+        const uint32_t sb = e4m3_encode(div_scale(div_six(amax[e]), g, rg));
         se[e] = e4m3_decode(sb) * g;
         s_scales[4 * lane + 2 * c + e][nb] = static_cast<uint8_t>(sb);
         ok = ok && se[e] > 1e-28f && se[e] < 1e28f && amax[e] < 1e28f;     // quotients of normal numbers (div2p)

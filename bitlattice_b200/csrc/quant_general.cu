@@ -113,13 +113,13 @@ __device__ __forceinline__ uint32_t e4m3_sr(float v, float u) {
 // Nearest codes and scale byte of a block of maximum am, the better of two block scales with four-over-six; t = scale * g.
 __device__ __forceinline__ void nearest_block(const GenArgs& A, const float v[16], float am, float g, uint32_t& sb, float& t,
                                               float& inv, uint2& codes) {
-  const float rg = __frcp_rn(g);
-  sb = e4m3_encode(div_rn(div_rn(am, 6.0f, 0.16666667163372039794921875f), g, rg));
+  const float rg = scale_rcp(g);
+  sb = e4m3_encode(div_scale(div_six(am), g, rg));
   t = e4m3_decode(sb) * g;
   inv = t > 0.0f ? __frcp_rn(t) : 0.0f;
   codes = e2m1_nearest16(v, inv);
   if (A.fos) {
-    const uint32_t sb4 = e4m3_encode(div_rn(am * 0.25f, g, rg));
+    const uint32_t sb4 = e4m3_encode(div_scale(am * 0.25f, g, rg));
     const float t4 = e4m3_decode(sb4) * g;
     const float inv4 = t4 > 0.0f ? __frcp_rn(t4) : 0.0f;
     const uint2 codes4 = e2m1_nearest16(v, inv4);
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kGenThreads) general_kernel(GenArgs A) {
       if (A.mode == BL_Q_SR) {
         const uint32_t idx0 = static_cast<uint32_t>(static_cast<uint64_t>(r) * static_cast<uint64_t>(A.cols) +
                                                     static_cast<uint64_t>(col0 + 16 * blk));
-        codes = e2m1_sr16(v, inv, A.key, idx0, sr_special(max_abs16_nan(v), inv));
+        codes = e2m1_sr16_any(v, inv, A.key, idx0);
       } else if (A.mode == BL_Q_EDEN) {
         float xx, xr;
         eden_sums(v, codes, t, xx, xr);
@@ -529,10 +529,8 @@ __global__ void __launch_bounds__(kGenThreads, 3) rotated_kernel(GenArgs A) {
       if (A.mode == BL_Q_SR) {
         const uint32_t idx = static_cast<uint32_t>(static_cast<uint64_t>(row0) * static_cast<uint64_t>(A.cols) +
                                                    static_cast<uint64_t>(col0 + 16 * b));
-        codes[0] = e2m1_sr16(va, inv[0], A.key, idx + static_cast<uint32_t>(pair[0]) * static_cast<uint32_t>(A.cols),
-                             sr_special(max_abs16_nan(va), inv[0]));
-        codes[1] = e2m1_sr16(vb, inv[1], A.key, idx + static_cast<uint32_t>(pair[1]) * static_cast<uint32_t>(A.cols),
-                             sr_special(max_abs16_nan(vb), inv[1]));
+        codes[0] = e2m1_sr16_any(va, inv[0], A.key, idx + static_cast<uint32_t>(pair[0]) * static_cast<uint32_t>(A.cols));
+        codes[1] = e2m1_sr16_any(vb, inv[1], A.key, idx + static_cast<uint32_t>(pair[1]) * static_cast<uint32_t>(A.cols));
       } else if (A.mode == BL_Q_EDEN) {
         float2 xx, xr;
         eden_sums2(v, codes, t, xx, xr);

@@ -376,3 +376,22 @@ def test_division_on_every_significand(slice_):
     bad = ctypes.c_uint64(1)
     _C.call("bl_selftest_division_slice", slice_, ctypes.byref(bad), 0)
     assert bad.value == 0
+
+
+@pytest.mark.parametrize("g", [1e-38, 1e-30, 1e-20, 9.9e-13, 1e-12, 2.5e27, 1e37])
+def test_block_scales_of_extreme_tensors(g):
+    """Block maxima from a zero and 2^80 below the tensor's up to it, against per-tensor scales on both sides of the range in
+    which the scales' divisions go by a shared reciprocal; rows and transposed, both roundings."""
+    rng = np.random.default_rng(31)
+    x = rng.standard_normal((256, 256)) * 2.0 ** rng.uniform(-80, 3, (16, 1, 16, 1)).repeat(16, 1).repeat(16, 3).reshape(256, 256) * 400.0
+    x = np.clip(x * g, -3e38, 3e38).astype(np.float32)
+    x[16:32, 32:48] = 0.0
+    gd = dev(np.array([g], np.float32))
+    for mode, seed in (("rtn", -1), ("sr", 11)):
+        rc, rs, _ = oracle.quantize_rows(x, np.float32(g), mode, seed=max(seed, 0))
+        packed, sc = _ops.quantize_nvfp4(dev(x), gd, seed=seed)
+        assert np.array_equal(host(sc), rs) and np.array_equal(host(packed), rc)
+        bound = min(np.float32(g), np.float32(1e35))
+        rc, rs = oracle.quantize_t(x, None, oracle.global_from_bound(float(bound)), mode, seed=max(seed, 0))
+        packed, sc, _ = _ops.quantize_nvfp4_t(dev(x), None, seed, 0, dev(np.array([bound], np.float32)))
+        assert np.array_equal(host(sc), rs) and np.array_equal(host(packed), rc)
