@@ -395,3 +395,24 @@ def test_block_scales_of_extreme_tensors(g):
         rc, rs = oracle.quantize_t(x, None, oracle.global_from_bound(float(bound)), mode, seed=max(seed, 0))
         packed, sc, _ = _ops.quantize_nvfp4_t(dev(x), None, seed, 0, dev(np.array([bound], np.float32)))
         assert np.array_equal(host(sc), rs) and np.array_equal(host(packed), rc)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_gates_at_the_ends_of_the_shared_reciprocal(dtype):
+    """Finite gates from -87 up share a warp with nothing else, so that every one of them takes the shared reciprocal; then the
+    same with one gate beyond in every thousand."""
+    bits = torch.arange(1 << 16, device="cuda", dtype=torch.int32).to(torch.int16).view(dtype)
+    g = bits[(bits.float() >= -87.0) & bits.float().isfinite()]
+    g = torch.cat([g, g[: -g.numel() % 256]])
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    u, da = (torch.randn(g.numel(), device="cuda", generator=gen).to(dtype) for _ in range(2))
+    mixed = g.clone()
+    mixed[::1000] = torch.tensor([-87.5, -88.0, -100.0, float("inf"), float("-inf"), float("nan")], device="cuda").to(dtype).repeat(g.numel())[: mixed[::1000].numel()]
+    for gate in (g, mixed):
+        gf, uf, df = gate.float(), u.float(), da.float()
+        d = 1.0 + torch.exp(-gf)
+        silu, sig = (gf / d).to(dtype).float(), 1.0 / d
+        want = ((silu * uf).to(dtype), ((df * uf).to(dtype).float() * sig * (1.0 + gf * (1.0 - sig))).to(dtype), (df * silu).to(dtype))
+        for a, b in zip((_ops.swiglu_fwd(gate, u), *_ops.swiglu_bwd(gate, u, da)), want):
+            nan = b.isnan()
+            assert torch.equal(a.isnan(), nan) and torch.equal(a.view(torch.int16)[~nan], b.view(torch.int16)[~nan])
