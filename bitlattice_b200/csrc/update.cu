@@ -911,6 +911,10 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
         }
       }
       ok = ok && s_new <= 4.0f * s_old && s_old <= 4.0f * s_new;
+      if (!ok) {      // values outside the unchecked divisions' range (zero gradients): before a projection in vain
+        update_group_general<PCB, DIR, GT>(T, r, cg, denom, div, use_div, lutAL, plut, P);
+        continue;
+      }
       // ---- projection back to (code, phase) (bitlattice/reference.py:250-274, 324-334)
       const uint32_t h0 = (T.offset + static_cast<uint32_t>(static_cast<uint64_t>(r) * cols + cg * 16)) * 0x27D4EB2Fu +
                           T.key;
@@ -941,7 +945,10 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
             (par == 0 ? pe[h] : po[h]) = p;
           }
         }
-        ok = ok && z < kUndecided;
+        if (z >= kUndecided) {                                  // rare: a draw next to its threshold
+          update_group_general<PCB, DIR, GT>(T, r, cg, denom, div, use_div, lutAL, plut, P);
+          continue;
+        }
         if constexpr (PCB == 4) pout = make_uint2(join_phases<4>(pe[0], po[0]), join_phases<4>(pe[1], po[1]));
         else pout = static_cast<PW>(join_phases<PCB>(pe[0], po[0]) | (join_phases<PCB>(pe[1], po[1]) << (8 * PCB)));
       } else {
@@ -973,10 +980,6 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
             phase_put<PCB>(pout, i + 8 * e, static_cast<uint32_t>(k) & pmask);
           }
         }
-      }
-      if (!ok) {      // rare: values outside the unchecked divisions' range, or a draw next to its threshold
-        update_group_general<PCB, DIR, GT>(T, r, cg, denom, div, use_div, lutAL, plut, P);
-        continue;
       }
       T.scales_out[r * scale_stride + cg] = static_cast<uint8_t>(sb_new);
       cout.x = e2m1_drop_negative_zero(cout.x);
