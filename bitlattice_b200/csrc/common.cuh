@@ -194,11 +194,13 @@ __device__ __forceinline__ float div_checked(float x, float y, float ry, float l
   ok = ok && aq > lo && aq < 1e30f;
   return fmaf(fmaf(-y, q0, x), ry, q0);
 }
-__device__ __forceinline__ float div_six(float x) {
+// div_rn for callers whose dividend is above 2^-100, or the quotient immaterial
+__device__ __forceinline__ float div_quotient(float x, float y, float ry) {
   bool ok = true;
-  const float q = div_checked(x, 6.0f, kInv6, 1e-30f, ok);
-  return __builtin_expect(ok, 1) ? q : div_general(x, 6.0f);
+  const float q = div_checked(x, y, ry, 1e-30f, ok);
+  return __builtin_expect(ok, 1) ? q : div_general(x, y);
 }
+__device__ __forceinline__ float div_six(float x) { return div_quotient(x, 6.0f, kInv6); }
 __device__ __forceinline__ float div_scale(float x, float g, float rg) {
   bool ok = true;
   const float q = div_checked(x, g, rg, kScaleQuotient, ok);

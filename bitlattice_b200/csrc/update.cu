@@ -899,9 +899,10 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
         const float SAT = sat0 + sat1, STT = stt0 + stt1;
         float rr = SAA > 0.0f ? SAT / SAA : 1.0f;
         rr = fminf(fmaxf(rr, P.r_lo), P.r_hi);
-        const uint32_t bits = e4m3_encode(div_rn(s_old * rr, gs, rgs));
+        // (s_old is above 2^-40 where this counts, and a quotient below 2^-9 becomes that)
+        const uint32_t bits = e4m3_encode(div_quotient(s_old * rr, gs, rgs));
         const float cand = e4m3_decode(bits) * gs;
-        const float q = div_rn(cand, s_old, inv_s);
+        const float q = div_quotient(cand, s_old, inv_s);
         const float before = STT - 2.0f * SAT + SAA;
         const float after = q * q * SAA - 2.0f * q * SAT + STT;
         if ((after <= before) && isfinite(cand) && cand > 0.0f && bits != sb_old) {
