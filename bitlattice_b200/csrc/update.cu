@@ -912,7 +912,9 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
         }
       }
       ok = ok && s_new <= 4.0f * s_old && s_old <= 4.0f * s_new;
-      if (!ok) {      // values outside the unchecked divisions' range (zero gradients): before a projection in vain
+      // Values outside the unchecked divisions' range (zero gradients) leave before a projection in vain, by a call of their own
+      // with colnorm: what would live across the projection with a common one is spilled. With sign hardly any do.
+      if (DIR == 3 && !ok) {
         update_group_general<PCB, DIR, GT>(T, r, cg, denom, div, use_div, lutAL, plut, P);
         continue;
       }
@@ -922,65 +924,69 @@ __global__ void __launch_bounds__(kThreads, 2) update_kernel(const __grid_consta
       const f32x2 nsnew2 = pk(-s_new, -s_new), rsnew2 = pk(inv_new, inv_new);
       uint2 cout = make_uint2(0u, 0u);
       PW pout{};
-      if constexpr (kNarrow) {
-        uint32_t z = 0u, pe[2], po[2];
+      bool decided = ok;
+      if (DIR == 2 || ok) {
+        if constexpr (kNarrow) {
+          uint32_t z = 0u, pe[2], po[2];
 #pragma unroll
-        for (int par = 0; par < 2; ++par) {                     // elements of even, then of odd index
-          uint32_t S[2][4], sg[2][4];
+          for (int par = 0; par < 2; ++par) {                     // elements of even, then of odd index
+            uint32_t S[2][4], sg[2][4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int i = 2 * k + par;
-            float t0, t1;
-            upk(div2p(mul2p(tau2[i], sold2), nsnew2, rsnew2), t0, t1);
-            project_pair(t0, t1, h0 + static_cast<uint32_t>(i) * 0x27D4EB2Fu, h0 + static_cast<uint32_t>(i + 8) * 0x27D4EB2Fu,
-                         spread, byte256, S[0][k], S[1][k], z);
-            sg[0][k] = __float_as_uint(t0);
-            sg[1][k] = __float_as_uint(t1);
+            for (int k = 0; k < 4; ++k) {
+              const int i = 2 * k + par;
+              float t0, t1;
+              upk(div2p(mul2p(tau2[i], sold2), nsnew2, rsnew2), t0, t1);
+              project_pair(t0, t1, h0 + static_cast<uint32_t>(i) * 0x27D4EB2Fu, h0 + static_cast<uint32_t>(i + 8) * 0x27D4EB2Fu,
+                           spread, byte256, S[0][k], S[1][k], z);
+              sg[0][k] = __float_as_uint(t0);
+              sg[1][k] = __float_as_uint(t1);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t c, p;
+              split_levels(S[h], sg[h], P.pb, half4, pmask4, c, p);
+              uint32_t& out = h == 0 ? cout.x : cout.y;
+              out = par == 0 ? c : out + c * 16u;
+              (par == 0 ? pe[h] : po[h]) = p;
+            }
           }
+          decided = ok && z < kUndecided;                         // (66 of 2^24 draws are too near their threshold)
+          if constexpr (PCB == 4) pout = make_uint2(join_phases<4>(pe[0], po[0]), join_phases<4>(pe[1], po[1]));
+          else pout = static_cast<PW>(join_phases<PCB>(pe[0], po[0]) | (join_phases<PCB>(pe[1], po[1]) << (8 * PCB)));
+        } else {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t c, p;
-            split_levels(S[h], sg[h], P.pb, half4, pmask4, c, p);
-            uint32_t& out = h == 0 ? cout.x : cout.y;
-            out = par == 0 ? c : out + c * 16u;
-            (par == 0 ? pe[h] : po[h]) = p;
+          for (int i = 0; i < 8; ++i) {
+            float tv[2];
+            upk(div2p(mul2p(tau2[i], sold2), nsnew2, rsnew2), tv[0], tv[1]);
+            // nearest levels of the pair through the hardware conversion (ties to even: see the notes above). It
+            // saturates, and beyond the last level the table's factor is 0, so a target outside [-6, 6] needs no clamp
+            // (the range check has made it finite): its phase coordinate is 0 either way.
+            const uint32_t near2 = cvt_e2m1x2(tv[1], tv[0]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const float t = tv[e];
+              const uint32_t nib = e == 0 ? (near2 & 15u) : (near2 >> 4);
+              const float4 L = plut24[nib];
+              // phase coordinate times half, in 2^-24 fixed point (exact scaling; |q| <= 64, so it fits 31 bits); the
+              // draw n = hash >> 8 rounds up iff n * 2^-24 < frac(q), i.e. iff n < ceil(frac(q) * 2^24): the carry of
+              // adding 2^24 - 1 - n to ceil(q * 2^24). k = floor(q) + carry, two's complement.
+              const int q24 = __float2int_ru((t - L.x) * (t < L.x ? L.z : L.y));
+              uint32_t h = h0 + static_cast<uint32_t>(i + 8 * e) * 0x27D4EB2Fu;
+              h = (h ^ (h >> 16)) * 0x7FEB352Du;
+              h = (h ^ (h >> 15)) * 0x846CA68Bu;
+              h = ~(h ^ (h >> 16));
+              const int k = (q24 + static_cast<int>(h >> 8)) >> 24;
+              const uint32_t code = k == half_i ? __float_as_uint(L.w) : nib;      // +half: the level above, phase -half
+              if (e == 0) cout.x += code << (4 * i);
+              else cout.y += code << (4 * i);
+              phase_put<PCB>(pout, i + 8 * e, static_cast<uint32_t>(k) & pmask);
+            }
           }
         }
-        if (z >= kUndecided) {                                  // rare: a draw next to its threshold
-          update_group_general<PCB, DIR, GT>(T, r, cg, denom, div, use_div, lutAL, plut, P);
-          continue;
-        }
-        if constexpr (PCB == 4) pout = make_uint2(join_phases<4>(pe[0], po[0]), join_phases<4>(pe[1], po[1]));
-        else pout = static_cast<PW>(join_phases<PCB>(pe[0], po[0]) | (join_phases<PCB>(pe[1], po[1]) << (8 * PCB)));
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float tv[2];
-          upk(div2p(mul2p(tau2[i], sold2), nsnew2, rsnew2), tv[0], tv[1]);
-          // nearest levels of the pair through the hardware conversion (ties to even: see the notes above). It
-          // saturates, and beyond the last level the table's factor is 0, so a target outside [-6, 6] needs no clamp
-          // (the range check has made it finite): its phase coordinate is 0 either way.
-          const uint32_t near2 = cvt_e2m1x2(tv[1], tv[0]);
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float t = tv[e];
-            const uint32_t nib = e == 0 ? (near2 & 15u) : (near2 >> 4);
-            const float4 L = plut24[nib];
-            // phase coordinate times half, in 2^-24 fixed point (exact scaling; |q| <= 64, so it fits 31 bits); the
-            // draw n = hash >> 8 rounds up iff n * 2^-24 < frac(q), i.e. iff n < ceil(frac(q) * 2^24): the carry of
-            // adding 2^24 - 1 - n to ceil(q * 2^24). k = floor(q) + carry, two's complement.
-            const int q24 = __float2int_ru((t - L.x) * (t < L.x ? L.z : L.y));
-            uint32_t h = h0 + static_cast<uint32_t>(i + 8 * e) * 0x27D4EB2Fu;
-            h = (h ^ (h >> 16)) * 0x7FEB352Du;
-            h = (h ^ (h >> 15)) * 0x846CA68Bu;
-            h = ~(h ^ (h >> 16));
-            const int k = (q24 + static_cast<int>(h >> 8)) >> 24;
-            const uint32_t code = k == half_i ? __float_as_uint(L.w) : nib;      // +half: the level above, phase -half
-            if (e == 0) cout.x += code << (4 * i);
-            else cout.y += code << (4 * i);
-            phase_put<PCB>(pout, i + 8 * e, static_cast<uint32_t>(k) & pmask);
-          }
-        }
+      }
+      if (!decided) {
+        update_group_general<PCB, DIR, GT>(T, r, cg, denom, div, use_div, lutAL, plut, P);
+        continue;
       }
       T.scales_out[r * scale_stride + cg] = static_cast<uint8_t>(sb_new);
       cout.x = e2m1_drop_negative_zero(cout.x);
