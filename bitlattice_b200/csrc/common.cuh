@@ -211,6 +211,13 @@ __device__ __forceinline__ float div_block_scale(float amax, float g, float rg, 
   return div_checked(div_checked(amax, 6.0f, kInv6, 1e-30f, ok), g, rg, kScaleQuotient, ok);
 }
 
+// 1 / x to within an ulp or so: a start for a correction, or a bracket
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // ---------------------------------------------------------------------------------------------- device: fp32 pairs
 // Two independent fp32 operations per instruction, each lane rounded to nearest like the scalar operation (the fused
 // multiply-add is written out only where a single rounding is wanted: the residuals of the divisions).
@@ -463,7 +470,7 @@ static __device__ __noinline__ uint32_t e2m1_sr8_exact(float4 x0, float4 x1, uin
 // with the additions that can be multiply-adds on the other pipe. At 65536 x 4096 bf16 on a B200: 311 -> 191 us for the row
 // quantizer, 472 -> 325 us for the transposed one. (The rounding conversion cvt.rs of this architecture draws from 8 bits per
 // element and cannot give the reference's codes.)
-static __device__ __constant__ uint32_t kPipeMul[2] = {1u << 10, 1u};   // from constant memory, so that products stay products
+static __device__ __constant__ uint32_t kPipeMul[1] = {1u << 10};   // from constant memory, so that the product stays a product
 
 __device__ __forceinline__ f32x2 mul2p_down(f32x2 a, f32x2 b) {            // rounded toward zero
   f32x2 r;

@@ -120,12 +120,6 @@ __device__ __forceinline__ int64_t scale_index(int layout, int64_t r, int64_t c1
 
 // ---- rows, one thread per block of 16 ---------------------------------------------------------------------------------
 
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 // block quantization modes
 constexpr int kModeRtn = 0, kModeSr = 1, kModeFosMse = 2, kModeFosMae = 3;
 
@@ -993,8 +987,9 @@ extern "C" int bl_nvfp4_amax(const void* x, int dtype, int64_t n, float* out, in
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   BL_CUDA(cudaMemsetAsync(out, 0, 16, st));
   // Four CTAs per SM with eight loads in flight per thread keep 128 KB under way on each and leave a quarter of the atomics
-  // at the end: 1903 x 4096 bf16 6.8 -> 4.6 us, 4096 x 4096 8.0 -> 5.7 us, 4999 x 25600 fp16 40.3 -> 38.9 us. From 256 MB on
-  // the end no longer counts and sixteen CTAs of single loads are 2 to 3 % ahead (65536 x 4096: 78 against 80 us).
+  // at the end. With the input in L2 (and from HBM): 1903 x 4096 bf16 7.3 -> 4.7 us (9.2 -> 7.4), 4096 x 4096 8.2 -> 5.8 us
+  // (12.4 -> 11.0), 4999 x 25600 fp16 40.6 -> 39.3 us (53.8 -> 52.9). From 256 MB on the end no longer counts and sixteen
+  // CTAs of single loads are 2 to 3 % ahead (65536 x 4096: 78 against 80 us).
   const int64_t vecs = n / (dtype == BL_F32 ? 4 : 8) + 1;
   const bool large = vecs >= (int64_t(1) << 24);
   const int64_t wave = static_cast<int64_t>(sm_count(device)) * (large ? 16 : 4), want = (vecs + kQThreads - 1) / kQThreads;

@@ -9,8 +9,8 @@
 //   4/6 error  per block: sequential sums over elements 4q .. 4q + 3, then (s0 + s1) + (s2 + s3)
 //   MS-EDEN    <x, x> and <x, x_rtn> per 128: sequential sums over 4 elements, then a pairwise tree (neighbours first)
 //
-// Thread mapping of general_kernel (unrotated operands; rotated_kernel below takes the others but an odd number of
-// transposed rows): a lane owns one 16-element block, eight neighbouring lanes one 128-element segment of an output row,
+// Thread mapping of general_kernel (unrotated operands, and rotated ones with an odd number of transposed rows; rotated_kernel
+// below takes the other rotated ones): a lane owns one 16-element block, eight neighbouring lanes one 128-element segment of an output row,
 // a warp four rows' segments at a time. Strides 1 .. 8 of the rotation run in registers, strides 16 .. 64 are shuffles
 // over lane distances 1, 2, 4; block scales, four-over-six errors and stochastic draws need no exchange, the MS-EDEN
 // sums three shuffle steps. A CTA covers 128 output columns x 64 output rows; for transposed output it first stages
@@ -216,8 +216,9 @@ __global__ void __launch_bounds__(kGenThreads) general_kernel(GenArgs A) {
   }
 
   const bool valid_col = col0 + 16 * blk < A.cols;         // cols is a multiple of 16: a whole block or none
+  const bool rotate = SRC == kSrcTransposed && A.rotate;   // (the others rotate in rotated_kernel)
   uint32_t neg = 0;                                        // bit i: the rotation negates element i of this lane
-  if (A.rotate) {
+  if (rotate) {
 #pragma unroll
     for (int i = 0; i < 16; ++i)
       neg |= (hash_uniform(static_cast<uint32_t>(16 * blk + i), A.rot_key) < 0.5f ? 1u : 0u) << i;
@@ -253,7 +254,7 @@ __global__ void __launch_bounds__(kGenThreads) general_kernel(GenArgs A) {
         for (int i = 0; i < 16; ++i) v[i] = tile[(16 * blk + i) * 65 + rr];
       }
     }
-    if (A.rotate) {
+    if (rotate) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ (((neg >> i) & 1u) << 31));
 #pragma unroll
@@ -622,8 +623,8 @@ static int general_typed(GenArgs A, bool packed, bool transpose, bool need_amax,
   const dim3 grid(static_cast<unsigned>((A.cols + 127) / 128), static_cast<unsigned>((A.rows + kGenTileRows - 1) / kGenTileRows));
   if (need_amax) BL_CUDA(cudaMemsetAsync(A.amax, 0, sizeof(float), st));
   // Rotated operands (cols is a multiple of 128): two rows at a time. Transposed ones read pairs of source columns, so
-  // their number must be even and the source aligned to a pair.
-  if (A.rotate && (!transpose || (A.rows % 2 == 0 && reinterpret_cast<uintptr_t>(A.x) % (2 * sizeof(T)) == 0))) {
+  // their number must be even.
+  if (A.rotate && (!transpose || A.rows % 2 == 0)) {
     constexpr unsigned kPer = kRotTiles * kGenTileRows;
     const dim3 rot(grid.x, static_cast<unsigned>((A.rows + kPer - 1) / kPer));
     for (int pass = need_amax ? 0 : 1; pass < 2; ++pass) {
@@ -648,8 +649,7 @@ static int general_typed(GenArgs A, bool packed, bool transpose, bool need_amax,
   }
   if (need_amax) {
     if (packed) general_kernel<uint8_t, kSrcPackedTransposed, 0><<<grid, kGenThreads, 0, st>>>(A);
-    else if (transpose) general_kernel<T, kSrcTransposed, 0><<<grid, kGenThreads, 0, st>>>(A);
-    else general_kernel<T, kSrcRows, 0><<<grid, kGenThreads, 0, st>>>(A);
+    else general_kernel<T, kSrcTransposed, 0><<<grid, kGenThreads, 0, st>>>(A);      // rotated, an odd number of rows
   }
   if (packed) general_kernel<uint8_t, kSrcPackedTransposed, 1><<<grid, kGenThreads, 0, st>>>(A);
   else if (transpose) general_kernel<T, kSrcTransposed, 1><<<grid, kGenThreads, 0, st>>>(A);

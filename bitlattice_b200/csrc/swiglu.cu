@@ -49,11 +49,6 @@ __device__ __forceinline__ void glu_backward(float g, float u, float da, float& 
 // out of line, as a whole (32768 x 12288 of N(0, 100^2): forward 1343 us by thread, 1130 by warp; gates that are all in range,
 // zeros among them or not, 401). The signs come out negated because the reciprocal's operand can be negated for free and
 // packed operands cannot.
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 __device__ __forceinline__ f32x2 newton_neg_rcp(float d0, float d1) {       // -1/d, two lanes
   const f32x2 nr = pk(rcp_approx(-d0), rcp_approx(-d1));
   return fma2p(nr, fma2p(pk(d0, d1), nr, pk(1.0f, 1.0f)), nr);
