@@ -465,10 +465,10 @@ static __device__ __noinline__ uint32_t e2m1_sr8_exact(float4 x0, float4 x1, uin
 // element that needs its low bits (2 of 2^16 sums, its eight elements then take e2m1_sr8_exact). A carry out of the last level
 // gives 8, which the conversion to E2M1 saturates to 6, as it does everything above 6.
 //
-// The loop is bound by the ALU pipe (shifts, bit operations, selects; 64 lanes per SM and clock): 8 such instructions per
-// element against 20 before -- no clamp, no float-to-integer conversion, no level look-up, no sign and nibble merging --
-// with the additions that can be multiply-adds on the other pipe. At 65536 x 4096 bf16 on a B200: 311 -> 191 us for the row
-// quantizer, 472 -> 325 us for the transposed one. (The rounding conversion cvt.rs of this architecture draws from 8 bits per
+// The loop is bound by issue (83 % of the slots in the row quantizer) beside the ALU pipe (shifts, bit operations, selects; 64
+// lanes per SM and clock; 77 %), which alone bound it before: 8 such instructions per element against 20 -- no clamp, no float-to-integer conversion, no level look-up, no sign and nibble merging --
+// with the additions that can be multiply-adds on the other pipe. At 65536 x 4096 bf16 on a B200: 310 -> 187 us for the row
+// quantizer, 468 -> 331 us for the transposed one. (The rounding conversion cvt.rs of this architecture draws from 8 bits per
 // element and cannot give the reference's codes.)
 static __device__ __constant__ uint32_t kPipeMul[1] = {1u << 10};   // from constant memory, so that the product stays a product
 

@@ -7,8 +7,8 @@
 // one thread handles 8 consecutive elements (16-byte accesses), grid-stride over the tensor, the next vectors' loads issued
 // before the current ones are worked on. What bounds it above the bytes is the arithmetic of the sigmoid: one exponential
 // and, in IEEE arithmetic, two divisions by the same d = 1 + exp(-g). glu_sigmoid shares one reciprocal between them. On a
-// B200, 65536 x 12288 bf16: forward 992 -> 841 us (5.7 TB/s), backward 1593 -> 1344 us (6.0 TB/s); 4096 x 12288: 77 -> 70
-// and 119 -> 95 us.
+// B200, 65536 x 12288 bf16: forward 986 -> 796 us (6.1 TB/s), backward 1585 -> 1325 us (6.1 TB/s); 4096 x 12288 from HBM: 70 ->
+// 59 and 106 -> 86 us.
 #include "common.cuh"
 
 namespace blb {

@@ -582,10 +582,11 @@ __device__ __forceinline__ bool in_range16(const float v[16], float lo, float hi
 // largest fraction sum: within 2^(2 + pb) + 1 <= 65 of the carry the truncated bits could matter, and the group takes the
 // general route (66 of 2^24 sums).
 //
-// What bounds the loop is the issue of instructions and their latency (16 warps on an SM, no pipe above 53 %): 66 per element
+// What bounds the loop is the issue of instructions and their latency (16 warps on an SM, no pipe above 58 %): 63 per element
 // against 83 when the projection found the nearest level by conversion, looked up 16 bytes by code and selected by side and
-// carry (shared-memory wavefronts 60 % then, 25 % now). With the lane tables and the prefetched rows: three decoder layers
-// (578.7 M weights, colnorm, 4 bits) 1960 -> 1455 us, 12288 x 4096 sign 155 -> 131 us, fp32 sign 2 bits 160 -> 135 us.
+// carry (shared-memory wavefronts 60 % then, 24 % now). With the lane tables and the prefetched rows: the step of three decoder
+// layers (578.7 M weights, colnorm, 4 bits, statistics included) 2260 -> 1528 us, 12288 x 4096 sign 155 -> 131 us, fp32 sign
+// 2 bits 160 -> 135 us.
 static __device__ __constant__ uint32_t kUpdateMul[1] = {256u};   // from constant memory, so that the product stays a product
 constexpr uint32_t kUndecided = 0u - (66u << 8);
 
