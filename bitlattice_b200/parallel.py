@@ -50,7 +50,7 @@ from collections import OrderedDict
 import torch
 import torch.distributed as dist
 
-from .tensor import _PLAIN, _no_overrides, LatticeTensor, wait_for_update
+from .tensor import _PLAIN, _all_plain, _no_overrides, LatticeTensor, wait_for_update
 
 __all__ = ["ColumnParallelFp4Linear", "ColumnParallelLinear", "GatheredWeights", "SharedInputFp4Linears",
            "TokenParallelFp4Linear", "TokenParallelLinear", "column_parallel_linear", "column_parallel_linears",
@@ -360,8 +360,10 @@ class SharedInputFp4Linears(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, *gys):
-        with _no_overrides():
-            return SharedInputFp4Linears._gradients(ctx, *gys)
+        if _all_plain(gys):
+            with _no_overrides():
+                return SharedInputFp4Linears._gradients(ctx, *gys)
+        return SharedInputFp4Linears._gradients(ctx, *gys)
 
     @staticmethod
     def _gradients(ctx, *gys):

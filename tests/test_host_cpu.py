@@ -235,3 +235,26 @@ def test_what_is_not_a_cuda_tensor_is_refused_by_name():
                            (lambda: _ops.nvfp4_gemm(bad, t, t, t, t, t), "a_packed")):
             with pytest.raises(RuntimeError, match=f"^{name} must be a CUDA tensor"):
                 call()
+
+
+def test_user_code_around_a_layer_keeps_its_operator_interception(monkeypatch):
+    """Interception is off inside a layer only: a bias of a tensor subclass still sees the operators that it takes part in, and
+    saved-tensor hooks run with interception on."""
+    w = cpu_weight()
+    monkeypatch.setattr(bl.LatticeTensor, "dequantize", lambda self, dtype=torch.float32: torch.ones(32, 64, dtype=dtype))
+    seen, states = [], []
+
+    class Watched(torch.Tensor):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", str(func)))
+            return super().__torch_function__(func, types, args, kwargs)
+
+    x = torch.randn(4, 64, requires_grad=True)
+    torch.nn.functional.linear(x, w, torch.zeros(32).as_subclass(Watched))
+    assert "linear" in seen
+    note = lambda t: (states.append(torch._C._is_torch_function_enabled()), t)[1]
+    with torch.autograd.graph.saved_tensors_hooks(note, note):
+        y = torch.nn.functional.linear(x, w)
+    y.sum().backward()
+    assert len(states) >= 2 and all(states)
