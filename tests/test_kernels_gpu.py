@@ -617,7 +617,7 @@ def test_gemm_rejects_bad_shapes():
 
 
 def test_shared_reciprocal_division_is_exact():
-    """The kernels' division routine (shared correctly-rounded reciprocal + two fused corrections) equals the plain
+    """The kernels' division routine (shared correctly-rounded reciprocal + one fused correction) equals the plain
     fp32 division bit for bit on 2^30 pseudo-random operand pairs."""
     import ctypes
     from bitlattice_b200 import _C
